@@ -79,12 +79,19 @@ double nl_boxes(const int dim[3], uint32_t nq, uint32_t np, double reach, int nb
 // none; a box's points are split evenly.
 void launch_frames_groups(const BatchGrid& g, uint32_t nboxes, uint4* items, uint32_t* n_items, cudaStream_t s);
 
-// The grid of one system of up to SMALL_N points by one block (fg_small_grid.cu), with its
-// query groups where items is set. Grids have at most 2 n + 64 cells, which fit the
-// block's shared memory and 16 bits. Up to there the block is the faster one, whole calls
+// The grid of one system of up to SMALL_N points and SMALL_CELLS cells by one block
+// (fg_small_grid.cu), with its query groups where items is set. A system's own grid has at
+// most 2 n + 64 cells, so its points decide; query points of their own are put into the cells of the
+// points' grid, which may be any number. Both limits together fit the block's shared memory
+// (131 KB) and 16 bits a cell. Up to there the block is the faster one, whole calls
 // against the general build: RDF of 1000 points 99 / 112 us, 6000 108 / 114, 10000 116 / 118;
 // Steinhardt 129 / 146, 136 / 148, 150 / 163; NeighborList 143 / 156, 184 / 186, 212 / 201.
 constexpr uint32_t SMALL_N = 8192;
+constexpr uint32_t SMALL_CELLS = 2 * SMALL_N + 64;
+inline bool small_grid_fits(uint32_t n, uint64_t ncell)
+{
+    return n <= SMALL_N && ncell <= SMALL_CELLS;
+}
 struct SmallGrid
 {
     FrameDesc F;         // box, dim, ncell; boxes of the query groups; cell_base 0

@@ -575,7 +575,7 @@ void build_grid(const DevBox& db, const float* dpts, uint32_t n, const int dim[3
     g.start.alloc(sizeof(uint32_t) * (g.ncell + 1));
     g.cpos.alloc(sizeof(float4) * n);
     g.cidx.alloc(sizeof(uint32_t) * n);
-    if (n <= SMALL_N)
+    if (small_grid_fits(n, g.ncell))
     {
         SmallGrid a {};
         a.F.b = db;
@@ -3657,7 +3657,7 @@ uint32_t* n_items(const BatchGridBufs& g)
 void enqueue_grid_build(fg_frames* fr, BatchGridBufs& g, cudaStream_t s, bool sorted, uint32_t nboxes)
 {
     const uint32_t F = static_cast<uint32_t>(fr->n.size());
-    if (F == 1 && fr->total <= SMALL_N)
+    if (F == 1 && small_grid_fits(fr->total, g.ncell))
     {
         SmallGrid a {};
         a.F = g.fd_host[0];
