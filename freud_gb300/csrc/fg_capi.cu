@@ -625,8 +625,9 @@ GridEntry& nq_grid(fg_nq* nq, const int dim[3], bool sorted = true)
     }
     if (nq->grids.size() >= 4)
         nq->grids.erase(nq->grids.begin());
-    nq->grids.push_back(std::make_unique<GridEntry>());
-    build_grid(nq->dbox, nq->dpts, nq->n, dim, *nq->grids.back(), sorted);
+    auto built = std::make_unique<GridEntry>(); // (kept only once its build is on the stream)
+    build_grid(nq->dbox, nq->dpts, nq->n, dim, *built, sorted);
+    nq->grids.push_back(std::move(built));
     return *nq->grids.back();
 }
 
@@ -898,11 +899,11 @@ GridEntry& nq_ghost_grid(fg_nq* nq, float r_cut)
     }
     if (nq->ghost_grids.size() >= 2)
         nq->ghost_grids.erase(nq->ghost_grids.begin());
-    nq->ghost_grids.push_back(std::make_unique<GridEntry>());
-    GridEntry& g = *nq->ghost_grids.back();
-    g.r_cut = r_cut;
-    build_ghost_grid(ghost_setup(nq->box, nq->dbox, r_cut), nq->dpts, nq->n, 1, g);
-    return g;
+    auto built = std::make_unique<GridEntry>();
+    built->r_cut = r_cut;
+    build_ghost_grid(ghost_setup(nq->box, nq->dbox, r_cut), nq->dpts, nq->n, 1, *built);
+    nq->ghost_grids.push_back(std::move(built));
+    return *nq->ghost_grids.back();
 }
 
 // Query points (the object's points when dq is NULL) in the cells of a ghost
@@ -3673,6 +3674,7 @@ void enqueue_grid_build(fg_frames* fr, BatchGridBufs& g, cudaStream_t s, bool so
         a.words = n_items(g);
         a.n_words = 1 + ST_MAX_NL;
         launch_small_grid(a, s);
+        FG_CUDA(cudaGetLastError()); // the kernels that follow read what it writes
         return;
     }
     FG_CUDA(cudaMemsetAsync(g.counts.p, 0, sizeof(uint32_t) * (g.ncell + 2 + ST_MAX_NL), s));

@@ -137,8 +137,11 @@ size_t small_grid_smem(uint32_t n, uint32_t ncell, bool sorted)
 void launch_small_grid(const SmallGrid& a, cudaStream_t s)
 {
     const size_t smem = small_grid_smem(a.n, a.F.ncell, a.sorted != 0);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_small_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    // more than 48 KB, static arrays included, has to be allowed; always the same limit, so that
+    // threads do not lower each other's
+    if (smem > 47 * 1024)
+        cudaFuncSetAttribute(k_small_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(small_grid_smem(SMALL_N, SMALL_CELLS, true)));
     ProfScope prof_("k_small_grid", s);
     k_small_grid<<<1, SG_T, smem, s>>>(a);
 }
