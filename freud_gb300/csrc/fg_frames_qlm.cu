@@ -1103,10 +1103,14 @@ int frame_row_floats(int l)
 
 uint64_t frame_segment_words(double groups, double bonds_per_point, uint32_t expected)
 {
-    // rows of a group: the most bonds of its 32 lanes, about three deviations above the mean
-    const double rows = bonds_per_point + 3.0 * std::sqrt(bonds_per_point) + 2.0;
+    // rows of a group (a segment's head is 3): while a group's bonds are summed once, the most bonds of its 32
+    // lanes, about three deviations above the mean; more bonds are summed in several sweeps, each
+    // with its own most, which add up to 2.1 (30 bonds a point), 2.4 (100) to 3.0 (270) times the
+    // mean of uniform points. Too few words run the call again: 1M points, 100 bonds, twice the work.
+    const double once = bonds_per_point + 3.0 * std::sqrt(bonds_per_point) + 5.0;
+    const double rows = bonds_per_point > 16.0 ? std::max(once, 3.1 * bonds_per_point) : once;
     const uint64_t slack = static_cast<uint64_t>(qlm_blocks<6, true>(expected)) * QW * SEG_CHUNK;
-    return static_cast<uint64_t>(groups * (SEG_HEAD + 32.0 * rows)) + slack;
+    return static_cast<uint64_t>(groups * 32.0 * rows) + slack;
 }
 
 void launch_frames_qlm(const BatchGrid& g, const BallParams& p, const FrameQlm& w, int k, cudaStream_t s)
