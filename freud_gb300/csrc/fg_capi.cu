@@ -1134,7 +1134,9 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
         }
         else
         {
-            gptr = &nq_grid(nq, dim);
+            // the plan holds the buffers of its own grid, which has the same cells where the box is
+            // some thousand times r_max; in any order, as the kernels a query at a time order their bonds
+            gptr = &nq_grid(nq, dim, !plan.used);
             if (!plan.used)
                 make_query_set(nq, *gptr, dq, nqp, qs);
         }
