@@ -415,6 +415,25 @@ struct GridEntry
     GhostParams gp {};
 };
 
+// A grid kept by a NeighborQuery. It does not change once it is built: a query holds it
+// (GridRef) until its work is done, while queries of other threads may look up or drop others, and waits
+// for the build where that is on another stream.
+struct SharedGrid : GridEntry
+{
+    cudaStream_t built_on = nullptr;
+    cudaEvent_t built = nullptr;
+    uint64_t used = 0; // when it was last looked up
+    SharedGrid() = default;
+    SharedGrid(const SharedGrid&) = delete;
+    SharedGrid& operator=(const SharedGrid&) = delete;
+    ~SharedGrid()
+    {
+        if (built != nullptr)
+            cudaEventDestroy(built);
+    }
+};
+using GridRef = std::shared_ptr<const SharedGrid>;
+
 struct fg_nq
 {
     HostBox box;
@@ -424,8 +443,10 @@ struct fg_nq
     uint32_t n;
     const float* dpts;
     DevBuf own;
-    std::vector<std::unique_ptr<GridEntry>> grids;
-    std::vector<std::unique_ptr<GridEntry>> ghost_grids; // CellQuery, per r_cut
+    std::mutex mu; // of the grids kept
+    uint64_t uses = 0;
+    std::vector<std::shared_ptr<SharedGrid>> grids;
+    std::vector<std::shared_ptr<SharedGrid>> ghost_grids; // CellQuery, per r_cut
 };
 
 struct fg_nlist
@@ -609,26 +630,48 @@ void build_grid(const DevBox& db, const float* dpts, uint32_t n, const int dim[3
     FG_CUDA(cudaGetLastError());
 }
 
-GridEntry& nq_grid(fg_nq* nq, const int dim[3], bool sorted = true)
+// The grid of a list for which match holds, the kept one or else the one that build makes; replace: a kept
+// one whose place it takes. At most most grids are kept, those looked up last.
+template<typename Match, typename Replace, typename Build>
+GridRef keep_grid(fg_nq* nq, std::vector<std::shared_ptr<SharedGrid>>& list, size_t most, Match&& match,
+                  Replace&& replace, Build&& build)
 {
-    // the grid used last is at the back (a query may hold two)
-    for (auto g = nq->grids.begin(); g != nq->grids.end(); ++g)
+    cudaStream_t s = stream();
+    std::lock_guard<std::mutex> lock(nq->mu);
+    for (auto& g : list)
     {
-        if ((*g)->dim[0] == dim[0] && (*g)->dim[1] == dim[1] && (*g)->dim[2] == dim[2])
+        if (match(*g))
         {
-            std::rotate(g, g + 1, nq->grids.end());
-            GridEntry& found = *nq->grids.back();
-            if (sorted && !found.sorted)
-                sort_grid(nq->n, found);
-            return found;
+            g->used = ++nq->uses;
+            if (g->built_on != s)
+                FG_CUDA(cudaStreamWaitEvent(s, g->built, 0));
+            return g;
         }
     }
-    if (nq->grids.size() >= 4)
-        nq->grids.erase(nq->grids.begin());
-    auto built = std::make_unique<GridEntry>(); // (kept only once its build is on the stream)
-    build_grid(nq->dbox, nq->dpts, nq->n, dim, *built, sorted);
-    nq->grids.push_back(std::move(built));
-    return *nq->grids.back();
+    auto g = std::make_shared<SharedGrid>();
+    build(*g);
+    FG_CUDA(cudaEventCreateWithFlags(&g->built, cudaEventDisableTiming));
+    FG_CUDA(cudaEventRecord(g->built, s));
+    g->built_on = s;
+    g->used = ++nq->uses;
+    auto at = std::find_if(list.begin(), list.end(), [&](const std::shared_ptr<SharedGrid>& e) { return replace(*e); });
+    if (at == list.end() && list.size() >= most)
+        at = std::min_element(list.begin(), list.end(), [](const std::shared_ptr<SharedGrid>& x,
+                                                           const std::shared_ptr<SharedGrid>& y) { return x->used < y->used; });
+    if (at != list.end())
+        *at = g;
+    else
+        list.push_back(g);
+    return g;
+}
+
+// The points in a grid of dims; sorted: each cell's by index.
+GridRef nq_grid(fg_nq* nq, const int dim[3], bool sorted = true)
+{
+    auto same = [&](const SharedGrid& g) { return g.dim[0] == dim[0] && g.dim[1] == dim[1] && g.dim[2] == dim[2]; };
+    return keep_grid(
+        nq, nq->grids, 4, [&](const SharedGrid& g) { return same(g) && (g.sorted || !sorted); }, same,
+        [&](SharedGrid& g) { build_grid(nq->dbox, nq->dpts, nq->n, dim, g, sorted); });
 }
 
 DevGrid view(const GridEntry& g)
@@ -890,20 +933,14 @@ Prefilter prefilter(const fg_nq* nq, int arith, const int dim[3], float r_max, f
 
 // The CellQuery ghost grid for r_cut (cached on the NeighborQuery; the
 // reference rebuilds it for every query, CellQuery.cc:26-30).
-GridEntry& nq_ghost_grid(fg_nq* nq, float r_cut)
+GridRef nq_ghost_grid(fg_nq* nq, float r_cut)
 {
-    for (auto& g : nq->ghost_grids)
-    {
-        if (g->r_cut == r_cut)
-            return *g;
-    }
-    if (nq->ghost_grids.size() >= 2)
-        nq->ghost_grids.erase(nq->ghost_grids.begin());
-    auto built = std::make_unique<GridEntry>();
-    built->r_cut = r_cut;
-    build_ghost_grid(ghost_setup(nq->box, nq->dbox, r_cut), nq->dpts, nq->n, 1, *built);
-    nq->ghost_grids.push_back(std::move(built));
-    return *nq->ghost_grids.back();
+    return keep_grid(
+        nq, nq->ghost_grids, 2, [&](const SharedGrid& g) { return g.r_cut == r_cut; }, [](const SharedGrid&) { return false; },
+        [&](SharedGrid& g) {
+            g.r_cut = r_cut;
+            build_ghost_grid(ghost_setup(nq->box, nq->dbox, r_cut), nq->dpts, nq->n, 1, g);
+        });
 }
 
 // Query points (the object's points when dq is NULL) in the cells of a ghost
@@ -939,6 +976,7 @@ struct NlPlan
     bool wrap = false, wide = false;
     int room = 0; // candidates that fit a group
     FrameDesc F;
+    GridRef grid;
     DevGrid g;
     QuerySet qs;
     NlGroups w {};
@@ -1001,9 +1039,9 @@ bool plan_nl_groups(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_arg
     P.F.n = nqp;
     float pd[3];
     nearest_plane(hb, pd);
-    GridEntry& g = nq_grid(nq, P.F.dim, false);
-    make_query_set(nq, g, dq, nqp, P.qs, false);
-    P.g = view(g);
+    P.grid = nq_grid(nq, P.F.dim, false);
+    make_query_set(nq, *P.grid, dq, nqp, P.qs, false);
+    P.g = view(*P.grid);
     const uint32_t nboxes = static_cast<uint32_t>(P.F.nb[0] * P.F.nb[1] * P.F.nb[2]);
     const size_t items = static_cast<size_t>(std::min(nboxes, nqp)) + nqp / 32 + 1;
     P.items.alloc(sizeof(uint4) * items);
@@ -1105,7 +1143,7 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
     }
     int dim[3];
     QuerySet qs;
-    GridEntry* gptr = nullptr;
+    GridRef gptr;
     BallParams p;
     p.r_max_sq = fmul(a.r_max, a.r_max);
     p.r_min_sq = fmul(a.r_min, a.r_min);
@@ -1126,7 +1164,7 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
     auto general_grid = [&] {
         if (arith == ARITH_GHOST)
         {
-            gptr = &nq_ghost_grid(nq, a.r_max);
+            gptr = nq_ghost_grid(nq, a.r_max);
             dim[0] = gptr->dim[0];
             dim[1] = gptr->dim[1];
             dim[2] = gptr->dim[2];
@@ -1134,9 +1172,9 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
         }
         else
         {
-            // the plan holds the buffers of its own grid, which has the same cells where the box is
-            // some thousand times r_max; in any order, as the kernels a query at a time order their bonds
-            gptr = &nq_grid(nq, dim, !plan.used);
+            // with a plan in any order (the kernels a query at a time order their bonds): where the box is
+            // some thousand times r_max it is the plan's own grid
+            gptr = nq_grid(nq, dim, !plan.used);
             if (!plan.used)
                 make_query_set(nq, *gptr, dq, nqp, qs);
         }
@@ -1161,7 +1199,7 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
     else
     {
         general_grid();
-        GridEntry& g = *gptr;
+        const GridEntry& g = *gptr;
         // candidate capacity per cell: 4096 for dense point sets, whose 27-cell stencils
         // would overflow 1024 and fall back to the warp-per-query kernels
         cap = cell_cap_for(view(g), nq->n, nq->box.is2d && arith != ARITH_GHOST);
@@ -1223,7 +1261,7 @@ void ball_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a
     }
     if (n_over > 0)
     {
-        GridEntry& g = *gptr;
+        const GridEntry& g = *gptr;
         BallParams po = p;
         po.nq = n_over;
         launch_ball_emit(nq->dbox, view(g), left.qpos, left.qidx, po, counts.as<uint32_t>(), offsets.as<uint64_t>(),
@@ -1275,7 +1313,8 @@ bool knn_by_groups(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args
         width = std::min(width, static_cast<double>(pd[2]) / dim[2]);
     width *= 1.0 - 1e-5;
     cudaStream_t s = stream();
-    GridEntry& g = nq_grid(nq, dim, false);
+    const GridRef grid = nq_grid(nq, dim, false);
+    const GridEntry& g = *grid;
     QuerySet qs;
     make_query_set(nq, g, dq, nqp, qs, false);
     FrameDesc F = frame_desc(hb, dim, 2);
@@ -1385,7 +1424,8 @@ void knn_nlist(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_args& a,
     }
     int dim[3];
     grid_dims(nq->box, static_cast<float>(width), nq->n, dim);
-    GridEntry& g = nq_grid(nq, dim);
+    const GridRef grid = nq_grid(nq, dim);
+    const GridEntry& g = *grid;
     QuerySet qs;
     make_query_set(nq, g, dq, nqp, qs);
     float pd[3];
@@ -1539,10 +1579,10 @@ CopyLane& copy_lane()
 
 // The object's own cell grid for a ball query of n points with arguments a (the grid that
 // ball_nlist looks up), built ahead of the query.
-void prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
+GridRef prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
 {
     if (a.mode != FG_MODE_BALL || nq->kind == FG_NQ_CELLQUERY)
-        return;
+        return nullptr;
     int dim[3];
     grid_dims(nq->box, a.r_max * (1.0f + 1e-5f), nq->n, dim);
     const int arith = nq->kind == FG_NQ_LINKCELL ? ARITH_WRAP : ARITH_AABB;
@@ -1550,29 +1590,30 @@ void prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
     double groups = 0.0, met = 0.0;
     if (g_count_kernel == 0 && (arith == ARITH_AABB || prefilter(nq, arith, dim, a.r_max, a.r_min).out2 > 0.0f) &&
         nl_group_grid(nq, a, n, F, groups, met))
-        nq_grid(nq, F.dim, false);
-    else
-        nq_grid(nq, dim);
+        return nq_grid(nq, F.dim, false);
+    return nq_grid(nq, dim);
 }
 
 // Copies n host query points to buf on the copy lane while the object's cell
 // grid for the query is built on the library stream; the library stream waits
 // for the copy before anything that follows. If the build fails, the copy is
-// waited for before the error leaves (the caller may release its points then).
-void upload_query_points(fg_nq* nq, const fg_query_args& a, const float* host, uint32_t n, DevBuf& buf)
+// waited for before the error leaves (the caller may release its points then). Returns the
+// grid, for the caller to hold until the build has been waited for.
+GridRef upload_query_points(fg_nq* nq, const fg_query_args& a, const float* host, uint32_t n, DevBuf& buf)
 {
     buf.alloc(sizeof(float) * 3 * static_cast<size_t>(n));
     if (n == 0)
-        return;
+        return nullptr;
     const cudaStream_t s = stream();
     CopyLane& c = copy_lane();
     FG_CUDA(cudaEventRecord(c.fork, s)); // the buffer's allocation is ordered on s
     FG_CUDA(cudaStreamWaitEvent(c.s, c.fork, 0));
     FG_CUDA(cudaMemcpyAsync(buf.p, host, sizeof(float) * 3 * static_cast<size_t>(n), cudaMemcpyHostToDevice, c.s));
     FG_CUDA(cudaEventRecord(c.join, c.s));
+    GridRef grid;
     try
     {
-        prebuild_ball_grid(nq, a, n);
+        grid = prebuild_ball_grid(nq, a, n);
     }
     catch (...)
     {
@@ -1581,6 +1622,7 @@ void upload_query_points(fg_nq* nq, const fg_query_args& a, const float* host, u
         throw;
     }
     FG_CUDA(cudaStreamWaitEvent(s, c.join, 0));
+    return grid;
 }
 
 // Whether n query points already on the device (dq) equal the object's points
@@ -1794,11 +1836,12 @@ fg_status fg_nq_query(fg_nq* nq, const float* query_points, uint32_t n_query, co
         require(args, "args");
         require(out, "out");
         DevBuf dq;
+        GridRef grid;
         const float* qp = nullptr;
         uint32_t nqp = nq->n;
         if (query_points != nullptr)
         {
-            upload_query_points(nq, checked_args(nq, args), query_points, n_query, dq);
+            grid = upload_query_points(nq, checked_args(nq, args), query_points, n_query, dq);
             if (!same_as_points(nq, dq.as<float>(), n_query))
             {
                 qp = dq.as<float>();
@@ -2321,10 +2364,10 @@ static void rdf_accumulate(fg_rdf* rdf, fg_nq* nq, const float* dq, uint32_t nqp
             }
             int dim[3];
             QuerySet qs;
-            GridEntry* gptr = nullptr;
+            GridRef gptr;
             if (arith == ARITH_GHOST)
             {
-                gptr = &nq_ghost_grid(nq, a.r_max);
+                gptr = nq_ghost_grid(nq, a.r_max);
                 dim[0] = gptr->dim[0];
                 dim[1] = gptr->dim[1];
                 dim[2] = gptr->dim[2];
@@ -2333,10 +2376,10 @@ static void rdf_accumulate(fg_rdf* rdf, fg_nq* nq, const float* dq, uint32_t nqp
             else
             {
                 grid_dims(nq->box, a.r_max * (1.0f + 1e-5f), nq->n, dim);
-                gptr = &nq_grid(nq, dim);
+                gptr = nq_grid(nq, dim);
                 make_query_set(nq, *gptr, dq, nqp, qs);
             }
-            GridEntry& g = *gptr;
+            const GridEntry& g = *gptr;
             BallParams p;
             p.r_max_sq = fmul(a.r_max, a.r_max);
             p.r_min_sq = fmul(a.r_min, a.r_min);

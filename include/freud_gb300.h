@@ -13,6 +13,10 @@
  * Host pointers are plain C arrays (float32 points are packed x,y,z triples, as
  * the reference's vec3<float>). Objects are opaque handles with explicit destroy.
  * Calls are synchronous: when a call returns, its results are complete.
+ *
+ * Threads: a host thread's calls run on a stream of its own (fg_set_stream names one for
+ * all). A NeighborQuery may be queried by several threads at once; any other object is used by one
+ * thread at a time, and an object is destroyed when no call uses it.
  */
 #ifndef FREUD_GB300_H
 #define FREUD_GB300_H
