@@ -1579,7 +1579,7 @@ CopyLane& copy_lane()
 
 // The object's own cell grid for a ball query of n points with arguments a (the grid that
 // ball_nlist looks up), built ahead of the query.
-GridRef prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
+GridRef prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, int by_distance, uint32_t n)
 {
     if (a.mode != FG_MODE_BALL || nq->kind == FG_NQ_CELLQUERY)
         return nullptr;
@@ -1588,7 +1588,8 @@ GridRef prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
     const int arith = nq->kind == FG_NQ_LINKCELL ? ARITH_WRAP : ARITH_AABB;
     FrameDesc F;
     double groups = 0.0, met = 0.0;
-    if (g_count_kernel == 0 && (arith == ARITH_AABB || prefilter(nq, arith, dim, a.r_max, a.r_min).out2 > 0.0f) &&
+    if (!by_distance && g_count_kernel == 0 &&
+        (arith == ARITH_AABB || prefilter(nq, arith, dim, a.r_max, a.r_min).out2 > 0.0f) &&
         nl_group_grid(nq, a, n, F, groups, met))
         return nq_grid(nq, F.dim, false);
     return nq_grid(nq, dim);
@@ -1599,7 +1600,8 @@ GridRef prebuild_ball_grid(fg_nq* nq, const fg_query_args& a, uint32_t n)
 // for the copy before anything that follows. If the build fails, the copy is
 // waited for before the error leaves (the caller may release its points then). Returns the
 // grid, for the caller to hold until the build has been waited for.
-GridRef upload_query_points(fg_nq* nq, const fg_query_args& a, const float* host, uint32_t n, DevBuf& buf)
+GridRef upload_query_points(fg_nq* nq, const fg_query_args& a, int by_distance, const float* host, uint32_t n,
+                            DevBuf& buf)
 {
     buf.alloc(sizeof(float) * 3 * static_cast<size_t>(n));
     if (n == 0)
@@ -1613,7 +1615,7 @@ GridRef upload_query_points(fg_nq* nq, const fg_query_args& a, const float* host
     GridRef grid;
     try
     {
-        grid = prebuild_ball_grid(nq, a, n);
+        grid = prebuild_ball_grid(nq, a, by_distance, n);
     }
     catch (...)
     {
@@ -1841,7 +1843,7 @@ fg_status fg_nq_query(fg_nq* nq, const float* query_points, uint32_t n_query, co
         uint32_t nqp = nq->n;
         if (query_points != nullptr)
         {
-            grid = upload_query_points(nq, checked_args(nq, args), query_points, n_query, dq);
+            grid = upload_query_points(nq, checked_args(nq, args), sort_by_distance, query_points, n_query, dq);
             if (!same_as_points(nq, dq.as<float>(), n_query))
             {
                 qp = dq.as<float>();
