@@ -190,7 +190,7 @@ class Box:
     @dimensions.setter
     def dimensions(self, value):
         assert value == 2 or value == 3
-        self._is2D = value == 2
+        self._is2D = bool(value == 2)
         self._set_L(self._L[0], self._L[1], self._L[2])
 
     @property
