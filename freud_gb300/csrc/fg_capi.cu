@@ -3523,8 +3523,8 @@ struct BatchGridBufs
     double groups = 0.0; // about how many query groups there are (uniform points)
     DevBuf items;  // query groups
     // one upload: [F] FrameDesc, then [F + 1] words each of cell_base, box_base and the
-    // frames' first points. The host copy lives until the stream has been waited for
-    // (calls wait before they return; the destructor does where one failed).
+    // frames' first points. The host copy lives until the stream has been waited for: pending is
+    // set from the copy to the end of the call (TablesCopied)
     std::vector<unsigned char> host_tables;
     cudaStream_t pending = nullptr;
     DevBuf tables;
@@ -3536,14 +3536,16 @@ struct BatchGridBufs
     // the kernels over them (ST_MAX_NL): one clear for all
     DevBuf counts, start, cell_of, rank, pos4, cpos0, cidx0, cpos, cidx, scan;
     DevBuf frame_out; // int per frame: some point outside the frame's box
-    BatchGridBufs() = default;
-    BatchGridBufs(const BatchGridBufs&) = delete;
-    BatchGridBufs& operator=(const BatchGridBufs&) = delete;
-    ~BatchGridBufs()
+    void wait_for_tables()
     {
         if (pending != nullptr)
             cudaStreamSynchronize(pending);
+        pending = nullptr;
     }
+    BatchGridBufs() = default;
+    BatchGridBufs(const BatchGridBufs&) = delete;
+    BatchGridBufs& operator=(const BatchGridBufs&) = delete;
+    ~BatchGridBufs() { wait_for_tables(); }
 };
 
 } // namespace
@@ -3567,6 +3569,29 @@ struct fg_frames
 };
 
 namespace {
+
+// At the end of a call on a batch no grid of it remembers the call's stream, which may be gone
+// when the batch is destroyed: done() where the stream has been waited for, else the destructor waits.
+class TablesCopied
+{
+public:
+    explicit TablesCopied(fg_frames* fr) : fr_(fr) {}
+    TablesCopied(const TablesCopied&) = delete;
+    TablesCopied& operator=(const TablesCopied&) = delete;
+    ~TablesCopied()
+    {
+        for (auto& g : fr_->grids)
+            g->wait_for_tables();
+    }
+    void done()
+    {
+        for (auto& g : fr_->grids)
+            g->pending = nullptr;
+    }
+
+private:
+    fg_frames* fr_;
+};
 
 // Most query groups that n points in the grid's boxes make.
 size_t max_items(const BatchGridBufs& g, uint32_t n)
@@ -4023,6 +4048,7 @@ static void rdf_frames(fg_rdf* rdf, fg_frames* fr, const fg_query_args& a)
                 return;
             }
         }
+        TablesCopied tables(fr); // (the tuner makes grids of its own)
         const BatchHistConfig cfg = tuned_config(fr, p, h, a.r_max);
         BatchGridBufs& g = batch_grid(fr, a.r_max, cfg.shell);
         const BatchGrid v = batch_view(fr, g);
@@ -4038,7 +4064,7 @@ static void rdf_frames(fg_rdf* rdf, fg_frames* fr, const fg_query_args& a)
         });
         FG_CUDA(cudaGetLastError());
         sync();
-        g.pending = nullptr;
+        tables.done();
         // F accumulate calls: the frame count grows by F, box and N are the last frame's
         rdf->frames += static_cast<uint32_t>(fr->n.size());
         rdf->box = fr->boxes.back();
@@ -4254,11 +4280,12 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         set_frame_orders(st, F, sys);
         return;
     }
+    TablesCopied tables(fr);
     BatchGridBufs& g = batch_grid(fr, a.r_max, 1);
     const BatchGrid v = batch_view(fr, g);
     if (steinhardt_by_l(st, fr, g, p, expect, max_rows, a, sys))
     {
-        g.pending = nullptr;
+        tables.done();
         set_frame_orders(st, F, sys);
         return;
     }
@@ -4368,7 +4395,7 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         FG_CUDA(cudaMemcpyAsync(sys.data(), fr->st_sys.p, sizeof(double) * sys.size(), cudaMemcpyDeviceToHost, s));
         sync();
     }
-    g.pending = nullptr;
+    tables.done();
     set_frame_orders(st, F, sys);
 }
 
