@@ -32,3 +32,14 @@ def test_bond_lists_fit(freud, bonds):
     n = 200000
     got = launches(freud, uniform(freud, n), (bonds / 4.18879) ** (1 / 3.0), 6, True)
     assert got["k_frames_qlm<LIST>"] == 1
+
+
+# averaging lists up to 64 neighbours a particle; the expected number decides, with four deviations
+@pytest.mark.parametrize("n", [600, 2000, 3072])
+@pytest.mark.parametrize("bonds, fits", [(14, True), (38, True), (41, False), (60, False), (113, False)])
+def test_small_averaged(freud, n, bonds, fits):
+    system = uniform(freud, n)
+    got = launches(freud, system, (bonds / 4.18879) ** (1 / 3.0), 6, True)
+    assert got.get("k_small_qlm", 0) == (1 if fits else 0)
+    # without averaging nothing is listed
+    assert launches(freud, system, (bonds / 4.18879) ** (1 / 3.0), 6, False).get("k_small_qlm", 0) == 1
