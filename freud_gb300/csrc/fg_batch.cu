@@ -141,11 +141,19 @@ template<bool FILL> struct FBWarp
 // same as with the two passes.
 constexpr uint32_t FB_CHUNK = 4096; // bond slots a warp takes at a time (one pass)
 
-template<bool FILL, bool ONE = false>
+// Cells of more than FB_HEAVY points would keep their warp busy long after the others are
+// done: the first launch lists their queries in groups of FB_PART and the second (LISTED) takes those,
+// a group a warp. W_l of 8192 points in one cell 1310 -> 13.6 ms, of a droplet of 8000 57 -> 4.9
+// ms (groups of 32: 17 and 6.5).
+constexpr uint32_t FB_HEAVY = 128;
+constexpr uint32_t FB_PART = 8; // queries of a listed group
+
+template<bool FILL, bool ONE, bool LISTED>
 __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
     k_frames_ball(BatchGrid g, BallParams p, uint32_t* __restrict__ counts, const uint64_t* __restrict__ offsets,
-                  uint32_t* __restrict__ bj, float4* __restrict__ bvd, uint32_t* __restrict__ seg = nullptr,
-                  unsigned long long* __restrict__ alloc = nullptr, unsigned long long cap = 0)
+                  uint32_t* __restrict__ bj, float4* __restrict__ bvd, uint32_t* __restrict__ seg,
+                  unsigned long long* __restrict__ alloc, unsigned long long cap, uint2* __restrict__ heavy,
+                  uint32_t* __restrict__ n_heavy)
 {
     __shared__ FBWarp<FILL> sw[FB_WARPS];
     const int lane = threadIdx.x & 31;
@@ -153,10 +161,11 @@ __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
     FBWarp<FILL>& W = sw[warp];
     const unsigned lt = (1u << lane) - 1u;
     const uint32_t nwarps = gridDim.x * FB_WARPS;
-    uint32_t c = blockIdx.x * FB_WARPS + warp;
-    if (c >= g.ncell)
+    uint32_t at = blockIdx.x * FB_WARPS + warp; // cell, or item of the list
+    const uint32_t work = LISTED ? *n_heavy : g.ncell;
+    if (at >= work)
         return;
-    uint32_t f = frame_of(g.cell_base, g.nframes, c);
+    uint32_t f = frame_of(g.cell_base, g.nframes, LISTED ? heavy[at].x : at);
     uint32_t qn = 0; // queued bonds (fill)
     unsigned long long cur = 0, cend = 0; // one pass: the warp's chunk [cur, cend)
 
@@ -178,19 +187,34 @@ __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
         __syncwarp();
     };
 
-    for (; c < g.ncell; c += nwarps)
+    for (; at < work; at += nwarps)
     {
+        const uint2 item = LISTED ? heavy[at] : make_uint2(at, 0u);
+        const uint32_t c = item.x;
         const uint32_t q0 = g.start[c];
-        const uint32_t nqc = g.start[c + 1] - q0;
+        const uint32_t nqc = LISTED ? min(g.start[c + 1] - q0, item.y + FB_PART) : g.start[c + 1] - q0;
         if (nqc == 0)
             continue;
-        if (c >= g.cell_base[f + 1])
+        if (!LISTED && nqc > FB_HEAVY)
+        {
+            const uint32_t groups = (nqc + FB_PART - 1) / FB_PART;
+            uint32_t to = 0;
+            if (lane == 0)
+                to = atomicAdd(n_heavy, groups);
+            to = __shfl_sync(FULL, to, 0);
+            for (uint32_t k = lane; k < groups; k += 32)
+                heavy[to + k] = make_uint2(c, FB_PART * k);
+            continue;
+        }
+        if (LISTED ? c < g.cell_base[f] || c >= g.cell_base[f + 1] : c >= g.cell_base[f + 1])
         {
             if (FILL && qn > 0)
             {
                 drain(qn);
                 qn = 0;
             }
+            if (LISTED)
+                f = frame_of(g.cell_base, g.nframes, c);
             while (c >= g.cell_base[f + 1])
                 ++f;
         }
@@ -240,7 +264,7 @@ __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
         const uint32_t T = W.it_off[27];
         const uint32_t ntile = (T + FB_TILE - 1) / FB_TILE;
 
-        for (uint32_t g0 = 0; g0 < nqc; g0 += 32)
+        for (uint32_t g0 = item.y; g0 < nqc; g0 += 32)
         {
             const uint32_t ng = min(32u, nqc - g0);
             uint32_t my_cnt = 0;          // bonds so far of query g0 + lane
@@ -261,7 +285,7 @@ __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
                 const uint32_t t0 = tile * FB_TILE;
                 const uint32_t TT = min(static_cast<uint32_t>(FB_TILE), T - t0);
                 // stage candidates [t0, t0 + TT) unless this tile is already staged
-                if (ntile > 1 || g0 == 0)
+                if (ntile > 1 || g0 == item.y)
                 {
                     __syncwarp();
                     for (uint32_t tl = lane; tl < TT; tl += 32)
@@ -458,6 +482,16 @@ __global__ void __launch_bounds__(FB_THREADS, FILL ? 8 : 10)
     }
     if (FILL && qn > 0)
         drain(qn);
+}
+
+__global__ void __launch_bounds__(256) k_fullest_cell(BatchGrid g, uint32_t* __restrict__ most)
+{
+    uint32_t m = 0;
+    for (uint32_t c = blockIdx.x * 256 + threadIdx.x; c < g.ncell; c += gridDim.x * 256)
+        m = max(m, g.start[c + 1] - g.start[c]);
+    m = __reduce_max_sync(FULL, m);
+    if ((threadIdx.x & 31) == 0 && m > 0)
+        atomicMax(most, m);
 }
 
 // ---------------------------------------------------------------------------
@@ -766,40 +800,65 @@ template<typename K> uint32_t frames_ball_blocks(K kernel, uint32_t ncell)
 }
 } // namespace
 
-void launch_frames_ball_count(const BatchGrid& g, const BallParams& p, uint32_t n, uint32_t* counts, cudaStream_t s)
+namespace {
+// The cells and then the groups of the heavy ones.
+template<bool FILL, bool ONE>
+void frames_ball(const char* name, const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                 uint32_t* counts, const uint64_t* offsets, uint32_t* bond_j, float4* bond_vd, uint32_t* seg,
+                 unsigned long long* alloc, uint64_t cap, cudaStream_t s)
 {
     if (n == 0 || g.ncell == 0)
         return;
-    const uint32_t blocks = frames_ball_blocks(k_frames_ball<false>, g.ncell);
-    ProfScope prof_("k_frames_ball<COUNT>", s);
-    k_frames_ball<false><<<blocks, FB_THREADS, 0, s>>>(g, p, counts, nullptr, nullptr, nullptr);
+    cudaMemsetAsync(heavy.n, 0, sizeof(uint32_t), s);
+    auto go = [&](auto kernel, const char* what, uint32_t items) {
+        ProfScope prof_(what, s);
+        kernel<<<frames_ball_blocks(kernel, items), FB_THREADS, 0, s>>>(g, p, counts, offsets, bond_j, bond_vd, seg, alloc,
+                                                                      cap, heavy.items, heavy.n);
+    };
+    go(k_frames_ball<FILL, ONE, false>, name, g.ncell);
+    if (n > FB_HEAVY)
+        go(k_frames_ball<FILL, ONE, true>, "k_frames_ball<LISTED>", static_cast<uint32_t>(ball_heavy_items(n)));
+}
+} // namespace
+
+void launch_fullest_cell(const BatchGrid& g, uint32_t* most, cudaStream_t s)
+{
+    ProfScope prof_("k_fullest_cell", s);
+    k_fullest_cell<<<grid_blocks(g.ncell, 256 * 4), 256, 0, s>>>(g, most);
 }
 
-void launch_frames_ball_fill(const BatchGrid& g, const BallParams& p, uint32_t n, const uint64_t* offsets,
-                             uint32_t* bond_j, float4* bond_vd, cudaStream_t s)
+size_t ball_heavy_items(uint32_t n)
 {
-    if (n == 0 || g.ncell == 0)
-        return;
-    const uint32_t blocks = frames_ball_blocks(k_frames_ball<true>, g.ncell);
-    ProfScope prof_("k_frames_ball<FILL>", s);
-    k_frames_ball<true><<<blocks, FB_THREADS, 0, s>>>(g, p, nullptr, offsets, bond_j, bond_vd);
+    return n / FB_PART + n / FB_HEAVY + 1;
 }
 
-uint64_t frames_ball_onepass_slack(uint32_t ncell)
+void launch_frames_ball_count(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                              uint32_t* counts, cudaStream_t s)
 {
-    // every warp may leave the rest of its last chunk unused
-    return static_cast<uint64_t>(frames_ball_blocks(k_frames_ball<true, true>, ncell)) * FB_WARPS * FB_CHUNK;
+    frames_ball<false, false>("k_frames_ball<COUNT>", g, p, n, heavy, counts, nullptr, nullptr, nullptr, nullptr, nullptr,
+                              0, s);
 }
 
-void launch_frames_ball_onepass(const BatchGrid& g, const BallParams& p, uint32_t n, uint32_t* counts, uint32_t* seg,
-                                uint32_t* bond_j, float4* bond_vd, unsigned long long* alloc, uint64_t cap,
-                                cudaStream_t s)
+void launch_frames_ball_fill(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                             const uint64_t* offsets, uint32_t* bond_j, float4* bond_vd, cudaStream_t s)
 {
-    if (n == 0 || g.ncell == 0)
-        return;
-    const uint32_t blocks = frames_ball_blocks(k_frames_ball<true, true>, g.ncell);
-    ProfScope prof_("k_frames_ball<ONE>", s);
-    k_frames_ball<true, true><<<blocks, FB_THREADS, 0, s>>>(g, p, counts, nullptr, bond_j, bond_vd, seg, alloc, cap);
+    frames_ball<true, false>("k_frames_ball<FILL>", g, p, n, heavy, nullptr, offsets, bond_j, bond_vd, nullptr, nullptr, 0,
+                             s);
+}
+
+uint64_t frames_ball_onepass_slack(uint32_t ncell, uint32_t n)
+{
+    // every warp of either launch may leave the rest of its last chunk unused
+    const uint64_t blocks = frames_ball_blocks(k_frames_ball<true, true, false>, ncell) +
+        (n > FB_HEAVY ? frames_ball_blocks(k_frames_ball<true, true, true>, static_cast<uint32_t>(ball_heavy_items(n))) : 0u);
+    return blocks * FB_WARPS * FB_CHUNK;
+}
+
+void launch_frames_ball_onepass(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                                uint32_t* counts, uint32_t* seg, uint32_t* bond_j, float4* bond_vd,
+                                unsigned long long* alloc, uint64_t cap, cudaStream_t s)
+{
+    frames_ball<true, true>("k_frames_ball<ONE>", g, p, n, heavy, counts, nullptr, bond_j, bond_vd, seg, alloc, cap, s);
 }
 
 int frames_sys_splits(uint32_t max_rows)

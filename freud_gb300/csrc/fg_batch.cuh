@@ -124,7 +124,7 @@ void launch_frames_hist(const BatchHistConfig& cfg, const BatchGrid& g, const Ba
 constexpr uint32_t SMALL_RDF_N = 5120;
 // Whether the nearest image of a pair is the one within r_max: no tilt, and r_max below half
 // of every length with room for the rounding.
-bool nearest_image_fits(const DevBox& b, float r_max);
+bool nearest_image_fits(const float L[3], bool tilted, bool is2d, float r_max);
 bool small_hist_fits(const DevBox& b, uint32_t n, float r_max, uint32_t bins);
 void launch_small_hist(const DevBox& b, const float* pts, uint32_t n, int exclude_ii, const HistParams& h,
                        unsigned long long* hist, cudaStream_t s);
@@ -133,17 +133,27 @@ void launch_small_hist(const DevBox& b, const float* pts, uint32_t n, int exclud
 // Count pass: counts[i] = bonds of point i. Fill pass: bonds of point i at
 // offsets[i] in candidate order: the neighbour index j and one float4 holding the
 // Steinhardt bond vector box.wrap(p_j - p_i) (Steinhardt.cc:155) and the distance.
-void launch_frames_ball_count(const BatchGrid& g, const BallParams& p, uint32_t n, uint32_t* counts, cudaStream_t s);
-void launch_frames_ball_fill(const BatchGrid& g, const BallParams& p, uint32_t n, const uint64_t* offsets,
-                             uint32_t* bond_j, float4* bond_vd, cudaStream_t s);
+// *most (zeroed) = points of the fullest cell.
+void launch_fullest_cell(const BatchGrid& g, uint32_t* most, cudaStream_t s);
+// heavy: room for ball_heavy_items(n) groups of cells of many points, and their number.
+struct BallHeavy
+{
+    uint2* items;
+    uint32_t* n;
+};
+size_t ball_heavy_items(uint32_t n);
+void launch_frames_ball_count(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                              uint32_t* counts, cudaStream_t s);
+void launch_frames_ball_fill(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                             const uint64_t* offsets, uint32_t* bond_j, float4* bond_vd, cudaStream_t s);
 // One pass without the counts: warps take chunks of the bond arrays (capacity
 // cap) from *alloc (zeroed before the launch); seg[i] / counts[i] = the first bond
 // of point i and its bond count, its bonds in candidate order. *alloc > cap after
 // the launch: the arrays were too small and nothing past cap was written.
-uint64_t frames_ball_onepass_slack(uint32_t ncell); // bond slots the chunk tails may leave unused
-void launch_frames_ball_onepass(const BatchGrid& g, const BallParams& p, uint32_t n, uint32_t* counts, uint32_t* seg,
-                                uint32_t* bond_j, float4* bond_vd, unsigned long long* alloc, uint64_t cap,
-                                cudaStream_t s);
+uint64_t frames_ball_onepass_slack(uint32_t ncell, uint32_t n); // bond slots the chunk tails may leave unused
+void launch_frames_ball_onepass(const BatchGrid& g, const BallParams& p, uint32_t n, const BallHeavy& heavy,
+                                uint32_t* counts, uint32_t* seg, uint32_t* bond_j, float4* bond_vd,
+                                unsigned long long* alloc, uint64_t cap, cudaStream_t s);
 
 // q_lm of every point from the ball query, for single l up to FRAME_QLM_MAX_L
 // (fg_frames_qlm.cu), with the neighbour averaging when list is set.

@@ -3566,6 +3566,7 @@ struct fg_frames
     DevBuf st_rows, st_rows_ave, st_head, st_segs; // single-l path (fg_frames_qlm.cu)
     GraphCache st_graph_a, st_graph_b, st_graph_one;
     DevBuf st_alloc; // one pass: bond slots taken
+    DevBuf st_heavy; // groups of cells of many points, after their number
 };
 
 namespace {
@@ -4093,17 +4094,54 @@ static void set_frame_orders(fg_steinhardt* st, uint32_t F, const std::vector<do
     st->computed = true;
 }
 
-// The frames' q_lm straight from the ball query, one l at a time (fg_frames_qlm.cu): for
-// up to six l of at most 12 without wl (its harmonics are float-float). Per l the query is
-// run again; against bond arrays shared by every l, 300,000 points at density 0.95, r_max
-// 1.5, with averaging: l = 6 0.44 -> 0.28 ms, l = 4, 6 0.83 -> 0.49 ms, l = 2, 4, 6, 8
-// 1.67 -> 0.94 ms (an l costs about 0.2 ms). Returns false where the bond arrays are to
-// be used.
+// What a ball query's q_lm without wl take, in microseconds, by every pair of a small system, by groups
+// one l at a time, and by bond arrays that every l shares with float-float harmonics: fits (5 to
+// 13 % rms) to whole calls of 500 to 200,000 uniform points in 1 to 256 frames, 1 to 6 l up to 12,
+// 7 to 113 bonds a point, averaged or not. The group kernels have the least work per point, but a
+// group is one warp's chain, again for every l; bond arrays are written by a warp a cell, whose chain is
+// long where few cells hold many points.
+struct SteinhardtTimes
+{
+    double pairs, by_l, arrays;
+};
+
+// Rounds of 32 candidates of a cell's warp: points in it, points in a cell around it.
+static double cell_rounds(double points, double around, bool flat)
+{
+    const double met = points + (flat ? 8.0 : 26.0) * around;
+    return points * std::ceil(met / 32.0) * (met > 128.0 ? 2.0 : 1.0);
+}
+
+static SteinhardtTimes steinhardt_times(const StLs& ls, bool average, double n, double cells, bool flat, double bonds)
+{
+    const double nl = ls.nl, max2 = static_cast<double>(ls.max_l) * ls.max_l;
+    double l2 = 0.0, orders = 0.0;
+    for (int k = 0; k < ls.nl; ++k)
+    {
+        l2 += static_cast<double>(ls.l[k]) * ls.l[k];
+        orders += ls.l[k] + 1.0;
+    }
+    const double per_cell = n / cells;
+    SteinhardtTimes t;
+    t.pairs = 79.0 + nl * (11.0 + 0.015 * n + 6.2e-7 * n * n);
+    t.by_l = 100.0 + nl * (27.0 + 0.086 * (flat ? 9.0 : 27.0) * per_cell + n * (1.0e-4 + 2.1e-5 * bonds)) +
+        l2 * bonds * (0.0085 + 1.0e-7 * n);
+    t.arrays = 140.0 + cell_rounds(per_cell, per_cell, flat) * (0.2 + 4.7e-5 * cells) + bonds * (2.0 + 0.018 * max2) +
+        n * (1.2e-3 + bonds * (5.0e-7 * max2 + 1.9e-6 * orders));
+    if (average)
+    {
+        t.pairs += nl * (9.8 + 0.061 * bonds);
+        t.by_l += 7.1 * nl + bonds * orders * (0.27 + 2.2e-6 * n);
+        t.arrays += 12.0 + 1.2e-6 * n * bonds * orders;
+    }
+    return t;
+}
+
+// The frames' q_lm straight from the ball query, one l at a time (fg_frames_qlm.cu), for which
+// the query is run again. Returns false where the bond lists do not fit.
 static bool steinhardt_by_l(fg_steinhardt* st, fg_frames* fr, BatchGridBufs& g, const BallParams& p, double expect,
                             uint32_t max_rows, const fg_query_args& a, std::vector<double>& sys)
 {
-    if (st->wl || st->st.nl > 6 || st->st.max_l > FRAME_QLM_MAX_L)
-        return false;
     cudaStream_t s = stream();
     const uint32_t P = fr->total;
     const uint32_t F = static_cast<uint32_t>(fr->n.size());
@@ -4187,25 +4225,25 @@ static bool steinhardt_by_l(fg_steinhardt* st, fg_frames* fr, BatchGridBufs& g, 
     }
 }
 
-// One small system without wl: every pair, no grid (launch_small_qlm). Returns false where
-// that does not apply, with outputs to be computed anew.
-static bool steinhardt_small(fg_steinhardt* st, fg_frames* fr, const BallParams& p, double expect, const fg_query_args& a,
-                             std::vector<double>& sys)
+// Whether one small system can do without a grid (launch_small_qlm; mean: expected bonds a particle).
+static bool steinhardt_pairs_fit(const fg_steinhardt* st, const fg_frames* fr, double mean, const fg_query_args& a)
 {
     // averaging needs every neighbour on its particle's list: the most of some thousand particles lie
     // about four deviations above the mean. (2000 particles, r_max 3: 549 us with the lists tried in vain
     // and the grid then, 464 at once.)
-    const double mean = expect / std::max<uint32_t>(fr->total, 1u);
     if (st->average && mean + 4.0 * std::sqrt(mean) > SMALL_ST_BONDS)
         return false;
-    // several l search the neighbours anew for each
-    if (fr->n.size() != 1 || fr->total > (st->st.nl == 1 ? SMALL_ST_N : SMALL_ST_N * 2 / 3) || st->wl || st->st.nl > 6 ||
-        st->st.max_l > FRAME_QLM_MAX_L)
-        return false;
+    const HostBox& b = fr->boxes[0];
+    return fr->n.size() == 1 && fr->total <= SMALL_ST_N &&
+        nearest_image_fits(b.L, b.xy != 0.0f || b.xz != 0.0f || b.yz != 0.0f, b.is2d, a.r_max);
+}
+
+// One small system: every pair, no grid. Returns false, with outputs to be computed anew, where a
+// particle's neighbours do not fit its list.
+static bool steinhardt_small(fg_steinhardt* st, fg_frames* fr, const BallParams& p, std::vector<double>& sys)
+{
     SmallQlm w {};
     w.b = make_devbox(fr->boxes[0]);
-    if (!nearest_image_fits(w.b, a.r_max))
-        return false;
     cudaStream_t s = stream();
     const size_t n = fr->total;
     size_t row = 0;
@@ -4281,15 +4319,69 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         expect += vol > 0.0 ? static_cast<double>(fr->n[f]) * fr->n[f] / vol * ball : 0.0;
     }
     std::vector<double> sys(2 * static_cast<size_t>(F) * stride);
-    if (steinhardt_small(st, fr, p, expect, a, sys))
+    // Up to six l of at most 12 without wl (its harmonics are float-float) go the way that comes out
+    // cheapest (steinhardt_times), bond arrays only where they do by an eighth: within 1 % of the
+    // best of the three on average. 2000 points,
+    // averaged, r_max 1.5: l = 6 by pairs 134 us, by l 169, arrays 199; l = 4, 6, 8, 10 287, 378, 227;
+    // 200,000 points, l = 4, 6, 8: by l 740, arrays 899; 5000 points, r_max 2.5, l = 2, 4, .., 12:
+    // by l 1490, arrays 730. Pairs are taken up to a fifth above the others where nothing is averaged: their time does
+    // not depend on where the points are, while a group or a cell of a cluster is a long chain.
+    const bool flat = fr->boxes[0].is2d;
+    const double mean = expect / std::max<uint32_t>(P, 1u);
+    const bool choose = !st->wl && st->st.nl <= 6 && st->st.max_l <= FRAME_QLM_MAX_L;
+    const bool pairs_fit = choose && steinhardt_pairs_fit(st, fr, mean, a);
+    if (pairs_fit)
     {
-        set_frame_orders(st, F, sys);
-        return;
+        int dim[3]; // of the grid that the other ways take
+        grid_dims(fr->boxes[0], a.r_max * (1.0f + 1e-5f), P, dim);
+        const SteinhardtTimes t = steinhardt_times(st->st, st->average, P, static_cast<double>(dim[0]) * dim[1] * dim[2], flat,
+                                                   mean);
+        if (t.pairs <= (st->average ? 1.0 : 1.2) * std::min(t.by_l, t.arrays) && steinhardt_small(st, fr, p, sys))
+        {
+            set_frame_orders(st, F, sys);
+            return;
+        }
     }
     TablesCopied tables(fr);
     BatchGridBufs& g = batch_grid(fr, a.r_max, 1);
     const BatchGrid v = batch_view(fr, g);
-    if (steinhardt_by_l(st, fr, g, p, expect, max_rows, a, sys))
+    bool precise = st->wl;   // float-float harmonics; also where the arrays are taken for their time
+    bool grid_built = false;
+    if (choose)
+    {
+        const SteinhardtTimes t = steinhardt_times(st->st, st->average, P, g.ncell, flat, mean);
+        if (st->average)
+        {
+            // (in clusters, too, the averaging over bond arrays is the faster one)
+            precise = 1.12 * t.arrays < t.by_l;
+        }
+        else if (1.12 * t.arrays + (F > 1 ? 80.0 : 20.0) < t.by_l)
+        {
+            // The fullest cell, read back, decides (12 to 20 us; with a batch, whose grid leaves the graph, 40): in a cluster the chain of its queries
+            // is as long as the groups' or longer (1000 points in one cell, l = 4, 6, 8: by pairs 0.2 ms,
+            // arrays 4.1; 8000 in a droplet, l = 4, 6: by l 1.3, arrays 4.9).
+            enqueue_grid_build(fr, g, s, true, 0);
+            grid_built = true;
+            fr->st_alloc.alloc(sizeof(unsigned long long));
+            FG_CUDA(cudaMemsetAsync(fr->st_alloc.p, 0, sizeof(uint32_t), s));
+            launch_fullest_cell(v, fr->st_alloc.as<uint32_t>(), s);
+            FG_CUDA(cudaGetLastError());
+            uint32_t most = 0;
+            FG_CUDA(cudaMemcpyAsync(&most, fr->st_alloc.p, sizeof(most), cudaMemcpyDeviceToHost, s));
+            sync();
+            const double around = static_cast<double>(P) / g.ncell;
+            const double uniform = around + 4.0 * std::sqrt(around) + 2.0; // fullest of uniform points
+            precise = most <= uniform ||
+                t.arrays + 0.2 * (cell_rounds(most, around, flat) - cell_rounds(uniform, around, flat)) < t.by_l;
+            if (!precise && pairs_fit && t.pairs < 2.0 * t.by_l && steinhardt_small(st, fr, p, sys))
+            {
+                tables.done();
+                set_frame_orders(st, F, sys);
+                return;
+            }
+        }
+    }
+    if (choose && !precise && steinhardt_by_l(st, fr, g, p, expect, max_rows, a, sys))
     {
         tables.done();
         set_frame_orders(st, F, sys);
@@ -4305,7 +4397,7 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
     auto enqueue_rest = [&](double mean_bonds) {
         launch_qlm(g.fd_host[0].b, fr->dpts, P, nullptr, nullptr, nullptr, fr->st_seg.as<uint32_t>(),
                    fr->st_counts.as<uint32_t>(), st->st, 0, st->qlm.as<float2>(), st->ql.as<float>(), s,
-                   fr->st_vd.as<float4>(), mean_bonds, st->wl ? 1 : 0);
+                   fr->st_vd.as<float4>(), mean_bonds, precise ? 1 : 0);
         const float2* src = st->qlm.as<float2>();
         const float* qn = st->ql.as<float>();
         if (st->average)
@@ -4326,21 +4418,24 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
     auto outputs_key = [&](std::vector<uint64_t> key) {
         for (const void* ptr : {fr->st_j.p, fr->st_vd.p, fr->st_seg.p, fr->st_counts.p, fr->st_partial.p, fr->st_sys.p,
                                 st->qlm.p, st->ql.p, st->qlm_ave.p, st->ql_ave.p, st->wlv.p, st->wl_terms.p,
-                                static_cast<void*>(st)})
+                                fr->st_heavy.p, static_cast<void*>(st)})
             key.push_back(reinterpret_cast<uint64_t>(ptr));
         for (uint64_t x : {fbits(a.r_max), fbits(a.r_min), static_cast<uint64_t>(a.exclude_ii),
                            static_cast<uint64_t>(st->average), static_cast<uint64_t>(st->wl),
-                           static_cast<uint64_t>(st->wl_normalize)})
+                           static_cast<uint64_t>(st->wl_normalize), static_cast<uint64_t>(precise),
+                           static_cast<uint64_t>(grid_built)})
             key.push_back(x);
         for (int k = 0; k < st->st.nl; ++k)
             key.push_back(static_cast<uint64_t>(st->st.l[k]));
         return key;
     };
+    fr->st_heavy.alloc(sizeof(uint2) * (1 + ball_heavy_items(P)));
+    const BallHeavy heavy {fr->st_heavy.as<uint2>() + 1, fr->st_heavy.as<uint32_t>()};
     bool done = false;
     // one pass: bonds placed by per-warp chunks, no counts beforehand; arrays sized by
     // the expected bonds or the last run's (whichever is larger) plus the chunk tails
     const uint64_t cap = static_cast<uint64_t>(std::max(1.25 * expect, 1.1 * static_cast<double>(st->bond_hint))) +
-                         frames_ball_onepass_slack(g.ncell) + P;
+                         frames_ball_onepass_slack(g.ncell, P) + P;
     if (cap < (1ull << 32))
     {
         fr->st_j.alloc(sizeof(uint32_t) * cap);
@@ -4349,9 +4444,10 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         std::vector<uint64_t> key = outputs_key({g.id, cap, reinterpret_cast<uint64_t>(fr->dpts),
                                                  reinterpret_cast<uint64_t>(fr->st_alloc.p)});
         run_graph(fr->st_graph_one, fr->graphs, key, "graph:steinhardt_frames", [&] {
-            enqueue_grid_build(fr, g, s, true, 0);
+            if (!grid_built)
+                enqueue_grid_build(fr, g, s, true, 0);
             FG_CUDA(cudaMemsetAsync(fr->st_alloc.p, 0, sizeof(unsigned long long), s));
-            launch_frames_ball_onepass(v, p, P, fr->st_counts.as<uint32_t>(), fr->st_seg.as<uint32_t>(),
+            launch_frames_ball_onepass(v, p, P, heavy, fr->st_counts.as<uint32_t>(), fr->st_seg.as<uint32_t>(),
                                        fr->st_j.as<uint32_t>(), fr->st_vd.as<float4>(),
                                        fr->st_alloc.as<unsigned long long>(), cap, s);
             enqueue_rest(expect / std::max<uint32_t>(P, 1));
@@ -4372,12 +4468,13 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         const std::vector<uint64_t> key_a = {g.id, reinterpret_cast<uint64_t>(fr->dpts),
                                              reinterpret_cast<uint64_t>(fr->st_counts.p),
                                              reinterpret_cast<uint64_t>(fr->st_offsets.p),
-                                             reinterpret_cast<uint64_t>(fr->st_scan.p), fbits(a.r_max), fbits(a.r_min),
+                                             reinterpret_cast<uint64_t>(fr->st_scan.p),
+                                             reinterpret_cast<uint64_t>(fr->st_heavy.p), fbits(a.r_max), fbits(a.r_min),
                                              static_cast<uint64_t>(a.exclude_ii)};
         run_graph(fr->st_graph_a, fr->graphs, key_a, "graph:steinhardt_frames_count", [&] {
             enqueue_grid_build(fr, g, s, true, 0);
             FG_CUDA(cudaMemsetAsync(fr->st_counts.p, 0, sizeof(uint32_t) * (P + 1), s));
-            launch_frames_ball_count(v, p, P, fr->st_counts.as<uint32_t>(), s);
+            launch_frames_ball_count(v, p, P, heavy, fr->st_counts.as<uint32_t>(), s);
             scan_u32_to_u64(fr->st_counts.as<uint32_t>(), fr->st_offsets.as<uint64_t>(), static_cast<size_t>(P) + 1,
                             fr->st_scan.p, s);
         });
@@ -4391,7 +4488,7 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         fr->st_vd.alloc(sizeof(float4) * std::max<uint64_t>(nb, 1));
         std::vector<uint64_t> key_b = outputs_key({g.id, nb, reinterpret_cast<uint64_t>(fr->st_offsets.p)});
         run_graph(fr->st_graph_b, fr->graphs, key_b, "graph:steinhardt_frames", [&] {
-            launch_frames_ball_fill(v, p, P, fr->st_offsets.as<uint64_t>(), fr->st_j.as<uint32_t>(),
+            launch_frames_ball_fill(v, p, P, heavy, fr->st_offsets.as<uint64_t>(), fr->st_j.as<uint32_t>(),
                                     fr->st_vd.as<float4>(), s);
             launch_segments_from_offsets(fr->st_counts.as<uint32_t>(), fr->st_offsets.as<uint64_t>(), P,
                                          fr->st_seg.as<uint32_t>(), s);

@@ -602,14 +602,14 @@ __global__ void __launch_bounds__(SM_WARPS * 32)
 
 } // namespace
 
-bool nearest_image_fits(const DevBox& b, float r_max)
+bool nearest_image_fits(const float L[3], bool tilted, bool is2d, float r_max)
 {
-    return !b.tilted && r_max < 0.499f * std::min(std::min(b.L[0], b.L[1]), b.is2d ? b.L[1] : b.L[2]);
+    return !tilted && r_max < 0.499f * std::min(std::min(L[0], L[1]), is2d ? L[1] : L[2]);
 }
 
 bool small_hist_fits(const DevBox& b, uint32_t n, float r_max, uint32_t bins)
 {
-    return n <= SMALL_RDF_N && bins <= HIST_WORDS_MAX && nearest_image_fits(b, r_max);
+    return n <= SMALL_RDF_N && bins <= HIST_WORDS_MAX && nearest_image_fits(b.L, b.tilted != 0, b.is2d != 0, r_max);
 }
 
 void launch_small_hist(const DevBox& b, const float* pts, uint32_t n, int exclude_ii, const HistParams& h,
