@@ -1858,6 +1858,8 @@ void qlm_flat(const DevBox& box, const float* pts, uint32_t n, const uint2* ij, 
 }
 } // namespace
 
+constexpr int FF2_SUMS = 48 * 1024; // most bytes of sums of a block of k_qlm_ff2
+
 // slots per thread of k_qlm_ff2: requested (l, m) with m of the larger parity count
 static size_t ff2_np(const StLs& ls)
 {
@@ -1905,11 +1907,13 @@ void launch_qlm(const DevBox& box, const float* pts, uint32_t n, const uint2* ij
             const int most = 200 * 1024;
             cudaFuncSetAttribute(k_qlm_ff<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
             cudaFuncSetAttribute(k_qlm_ff<32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+            // (48 KB of sums beside the static arrays pass what a block has without asking)
+            cudaFuncSetAttribute(k_qlm_ff2<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, FF2_SUMS);
             configured = true;
         }
         // four bonds per pass: four independent recurrence chains per step
         // (0.85 ms against 0.99 ms with two on the 256,000-point FCC set, l = 4..12)
-        if (ff2_np(ls) * 64 * sizeof(float4) <= 48 * 1024)
+        if (ff2_np(ls) * 64 * sizeof(float4) <= FF2_SUMS)
         {
             // two threads per particle (orders by parity): twice the particles per SM, packed
             const uint32_t blocks2 = (n + 31) / 32;
