@@ -391,9 +391,15 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS)
         const float cull2 = F.cull2;
         uint32_t nz = 0, nn = 0; // buffered candidates
         Q.own = half || (qout && p.exclude_ii) ? slot + 1 : 0u;
-        // whole stencil, queries in the box: each meets itself once, at distance 0
-        if (p.exclude_ii && !half && !qout && part == 0 && counted<LOW>(h, 0.0f) && lane == 0)
-            atomicAdd(hist + exact_bin(h, 0.0f), 0ull - it.w);
+        // whole stencil, queries in the box: each meets itself once, at distance 0 (coordinates that
+        // are not finite, which come with image 0, at none)
+        if (p.exclude_ii && !half && !qout && part == 0 && counted<LOW>(h, 0.0f))
+        {
+            const float self = dot3(__fsub_rn(Q.p.x, Q.p.x), __fsub_rn(Q.p.y, Q.p.y), __fsub_rn(Q.p.z, Q.p.z));
+            const unsigned met = __ballot_sync(GR_FULL, live && self == 0.0f);
+            if (lane == 0)
+                atomicAdd(hist + exact_bin(h, 0.0f), 0ull - __popc(met));
+        }
         // one site each for the next chunk of the stencil, the next round of 32 candidates
         // and the two sweeps (a buffer is swept once it holds 32, and at the end); of
         // several parts each takes every parts-th round
