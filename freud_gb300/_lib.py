@@ -51,6 +51,7 @@ SIGNATURES = {
     "fg_last_error": [],
     "fg_version": [],
     "fg_set_stream": [P],
+    "fg_release_memory": [],
     "fg_launch_count": [pu64],
     "fg_profile_enable": [i32],
     "fg_profile_report": [ctypes.c_char_p, ctypes.c_size_t],
@@ -195,6 +196,11 @@ def set_count_kernel(which):
 
 def set_stream(stream_ptr):
     check(lib.fg_set_stream(ctypes.c_void_p(stream_ptr) if stream_ptr else None))
+
+
+def release_memory():
+    """Give the device memory that the library keeps for reuse back to the driver."""
+    check(lib.fg_release_memory())
 
 
 def make_args(mode=MODE_NONE, num_neighbors=DEFAULT_NUM_NEIGHBORS, r_max=-1.0, r_min=0.0, r_guess=-1.0,

@@ -71,28 +71,16 @@ static void index_error(const std::string& m)
 static cudaStream_t g_user_stream = nullptr;
 static bool g_user_stream_set = false;
 
-static cudaStream_t stream()
-{
-    if (g_user_stream_set)
-        return g_user_stream;
-    static thread_local cudaStream_t own = nullptr;
-    static thread_local int own_dev = -1;
-    int dev = 0;
-    FG_CUDA(cudaGetDevice(&dev));
-    if (own == nullptr || own_dev != dev)
-    {
-        FG_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
-        own_dev = dev;
-    }
-    return own;
-}
+static cudaStream_t stream();
 
-// Device blocks kept for reuse. A released block goes to the free list of its device,
-// the releasing call's stream and its size class, and the next request of that class on
-// that stream takes it: its earlier work is on the same stream, or was waited for (every
-// entry point synchronises before it returns). At most CACHE_MAX bytes are kept per
-// device: all of them go back to the driver when a block would pass that, and when an
-// allocation fails. cudaMallocAsync alone cost a small call (about 30 buffers) a third of its time,
+// Device blocks kept for reuse. A released block goes to the free list of its device, the
+// releasing call's stream and its size class, and the next request of that class on that
+// stream takes it: its earlier work is on the same stream, or was waited for (every entry point
+// waits for its stream before it returns, also with an error). The blocks of a stream that is
+// used no more - its thread has ended, or the caller named another - are any stream's. At most a quarter of
+// a device's memory is kept: the blocks released longest ago go back to the driver's pool, which
+// holds on to half of the device's memory at most, all of them when an allocation fails, and everything
+// with fg_release_memory. cudaMallocAsync alone cost a small call (about 30 buffers) a third of its time,
 // and its pool remapped memory whenever two large lists were alive in turn: 3.2 ms
 // instead of 2.1 for a list of 115 M bonds and its RDF.
 class BlockCache
@@ -117,14 +105,21 @@ public:
     {
         {
             std::lock_guard<std::mutex> lock(mu_);
-            auto it = free_.find(Key {dev, s, bytes});
-            if (it != free_.end() && !it->second.empty())
+            for (const Key& key : {Key {dev, false, s, bytes}, Key {dev, true, nullptr, bytes}})
             {
-                void* p = it->second.back();
-                it->second.pop_back();
-                kept_[dev] -= bytes;
-                return p;
+                auto it = free_.find(key);
+                if (it != free_.end() && !it->second.empty())
+                {
+                    void* p = it->second.back().p;
+                    it->second.pop_back();
+                    kept_[dev] -= bytes;
+                    return p;
+                }
             }
+        }
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            limit(dev);
         }
         void* p = nullptr;
         cudaError_t e = cudaMallocAsync(&p, bytes, s);
@@ -141,56 +136,162 @@ public:
     // (may throw std::bad_alloc, the block then still the caller's)
     void put(void* p, size_t bytes, int dev, cudaStream_t s)
     {
-        if (bytes > CACHE_MAX)
-        {
-            cudaFreeAsync(p, s);
-            return;
-        }
-        bool full = false;
+        std::vector<void*> old;
         {
             std::lock_guard<std::mutex> lock(mu_);
-            full = kept_[dev] + bytes > CACHE_MAX;
+            const size_t most = limit(dev);
+            // room by this stream's blocks and those of no stream; work of other streams may
+            // still use theirs
+            while (kept_[dev] + bytes > most)
+            {
+                auto at = free_.end();
+                for (auto it = free_.begin(); it != free_.end(); ++it)
+                {
+                    const Key& k = it->first;
+                    if (!it->second.empty() && std::get<0>(k) == dev && (std::get<1>(k) || std::get<2>(k) == s) &&
+                        (at == free_.end() || it->second.front().released < at->second.front().released))
+                        at = it;
+                }
+                if (at == free_.end())
+                    break;
+                old.push_back(at->second.front().p);
+                at->second.erase(at->second.begin());
+                kept_[dev] -= std::get<3>(at->first);
+            }
+            if (kept_[dev] + bytes > most)
+            {
+                old.push_back(p);
+            }
+            else
+            {
+                free_[Key {dev, false, s, bytes}].push_back({p, ++clock_});
+                kept_[dev] += bytes;
+            }
         }
-        if (full)
-            give_back(dev); // sizes or streams of the past hold the room
-        std::lock_guard<std::mutex> lock(mu_);
-        free_[Key {dev, s, bytes}].push_back(p);
-        kept_[dev] += bytes;
+        for (void* q : old)
+            cudaFreeAsync(q, s);
     }
 
-private:
-    static constexpr size_t CACHE_MAX = size_t(24) << 30;
-    using Key = std::tuple<int, cudaStream_t, size_t>;
+    // No work of stream s is left, nor will there be any.
+    void leave(cudaStream_t s)
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (auto it = free_.begin(); it != free_.end();)
+        {
+            const Key k = it->first;
+            if (std::get<1>(k) || std::get<2>(k) != s)
+            {
+                ++it;
+                continue;
+            }
+            auto& to = free_[Key {std::get<0>(k), true, nullptr, std::get<3>(k)}];
+            std::vector<Block> both(to.size() + it->second.size());
+            std::merge(to.begin(), to.end(), it->second.begin(), it->second.end(), both.begin(),
+                       [](const Block& x, const Block& y) { return x.released < y.released; });
+            to = std::move(both);
+            it = free_.erase(it);
+        }
+    }
 
-    // Frees every kept block of the current device.
+    // Frees every kept block of the current device, and what its pool holds on to.
     void give_back(int dev)
     {
         std::vector<void*> blocks;
         {
             std::lock_guard<std::mutex> lock(mu_);
-            for (auto& f : free_)
+            for (auto it = free_.begin(); it != free_.end();)
             {
-                if (std::get<0>(f.first) != dev)
+                if (std::get<0>(it->first) != dev)
+                {
+                    ++it;
                     continue;
-                blocks.insert(blocks.end(), f.second.begin(), f.second.end());
-                f.second.clear();
+                }
+                for (const Block& b : it->second)
+                    blocks.push_back(b.p);
+                it = free_.erase(it);
             }
             kept_[dev] = 0;
         }
         cudaDeviceSynchronize();
         for (void* p : blocks)
             cudaFree(p);
+        cudaMemPool_t pool;
+        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, 0);
+    }
+
+private:
+    // device, of no stream, stream, bytes
+    using Key = std::tuple<int, bool, cudaStream_t, size_t>;
+    struct Block
+    {
+        void* p;
+        uint64_t released;
+    };
+
+    // Bytes kept of a device; its pool is told what to hold on to the first time (mu_ held).
+    size_t limit(int dev)
+    {
+        auto it = limit_.find(dev);
+        if (it != limit_.end())
+            return it->second;
+        size_t left = 0, total = 0;
+        if (cudaMemGetInfo(&left, &total) != cudaSuccess)
+            total = 0;
+        cudaMemPool_t pool;
+        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+        {
+            uint64_t hold = total / 2;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &hold);
+        }
+        return limit_.emplace(dev, total / 4).first->second;
     }
 
     std::mutex mu_;
-    std::map<Key, std::vector<void*>> free_;
-    std::map<int, size_t> kept_;
+    std::map<Key, std::vector<Block>> free_; // the front was released longest ago
+    std::map<int, size_t> kept_, limit_;
+    uint64_t clock_ = 0;
 };
 
 static BlockCache& block_cache()
 {
     static BlockCache* c = new BlockCache; // never destroyed: buffers may be released at exit
     return *c;
+}
+
+// The stream of a thread's calls; when the thread ends, its blocks are any stream's.
+struct OwnStream
+{
+    cudaStream_t s = nullptr;
+    int dev = -1;
+    ~OwnStream()
+    {
+        if (s != nullptr && cudaStreamSynchronize(s) == cudaSuccess)
+        {
+            try
+            {
+                block_cache().leave(s);
+            }
+            catch (...)
+            {
+            }
+        }
+    }
+};
+
+static cudaStream_t stream()
+{
+    if (g_user_stream_set)
+        return g_user_stream;
+    static thread_local OwnStream own;
+    int dev = 0;
+    FG_CUDA(cudaGetDevice(&dev));
+    if (own.s == nullptr || own.dev != dev)
+    {
+        FG_CUDA(cudaStreamCreateWithFlags(&own.s, cudaStreamNonBlocking));
+        own.dev = dev;
+    }
+    return own.s;
 }
 
 // Stream-ordered device buffer of at least the requested size.
@@ -513,9 +614,26 @@ struct fg_steinhardt
 
 namespace {
 
+// Waits for what a call that failed has left on its stream (its buffers are reused, its
+// caller's released, as after one that did not).
+void wait_after_error()
+{
+    try
+    {
+        const cudaStream_t s = stream();
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone)
+            cudaStreamSynchronize(s);
+    }
+    catch (...)
+    {
+    }
+}
+
 // Runs f, mapping exceptions to status codes.
 template<typename F> fg_status guard(F&& f)
 {
+    fg_status code = FG_ERR_RUNTIME;
     try
     {
         f();
@@ -524,18 +642,19 @@ template<typename F> fg_status guard(F&& f)
     catch (const Error& e)
     {
         g_last_error = e.what();
-        return e.code;
+        code = e.code;
     }
     catch (const std::bad_alloc&)
     {
         g_last_error = "host allocation failed";
-        return FG_ERR_MEMORY;
+        code = FG_ERR_MEMORY;
     }
     catch (const std::exception& e)
     {
         g_last_error = e.what();
-        return FG_ERR_RUNTIME;
     }
+    wait_after_error();
+    return code;
 }
 
 void require(const void* p, const char* what)
@@ -1758,8 +1877,20 @@ int fg_version(void)
 fg_status fg_set_stream(void* cuda_stream)
 {
     return guard([&] {
-        g_user_stream = static_cast<cudaStream_t>(cuda_stream);
+        const cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
+        if (g_user_stream_set && g_user_stream != s)
+            block_cache().leave(g_user_stream); // (calls waited for it; it may be gone)
+        g_user_stream = s;
         g_user_stream_set = cuda_stream != nullptr;
+    });
+}
+
+fg_status fg_release_memory(void)
+{
+    return guard([&] {
+        int dev = 0;
+        FG_CUDA(cudaGetDevice(&dev));
+        block_cache().give_back(dev);
     });
 }
 

@@ -81,8 +81,14 @@ typedef struct fg_frames fg_frames;
 /* Library */
 const char* fg_last_error(void);
 int fg_version(void);
-/* Stream the library launches on (a cudaStream_t); NULL restores the library's own. */
+/* Stream the library launches on (a cudaStream_t), for every thread; NULL restores the
+ * library's own. No call of another thread is under way. The stream lives until another one is set or
+ * the last call on it has returned. */
 fg_status fg_set_stream(void* cuda_stream);
+/* Device memory that released buffers left for reuse (at most a quarter of the device's, and half
+ * with what the driver's pool holds on to) back to the driver, for other users of the device. No
+ * call of another thread is under way. */
+fg_status fg_release_memory(void);
 
 /* Kernel launch accounting and per-kernel device timing (no counterpart in the
  * reference, which has no device code). fg_launch_count: kernels launched by
