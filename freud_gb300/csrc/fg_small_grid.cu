@@ -14,15 +14,18 @@ namespace {
 
 constexpr int SG_T = 1024;
 
+__device__ __forceinline__ uint32_t sort_size(uint32_t n)
+{
+    return n <= 64 ? 64u : 1u << (32 - __clz(n - 1));
+}
+
 // Ascending bitonic sort of n words in shared memory by the block, in its all-ascending form (a merge
 // opens by comparing each element with its mirror): elements past n count as the largest. Neighbouring
 // 32 pairs stay within 64 words while the pairs are at most 32 apart, so such stages need no
 // barrier of the block.
 __device__ __forceinline__ void block_sort(uint32_t* v, uint32_t n, uint32_t tid)
 {
-    uint32_t np = 64;
-    while (np < n)
-        np <<= 1;
+    const uint32_t np = sort_size(n);
     for (uint32_t k = 2; k <= np; k <<= 1)
     {
         for (uint32_t j = k >> 1; j > 0; j >>= 1)
@@ -50,10 +53,11 @@ __device__ __forceinline__ void block_sort(uint32_t* v, uint32_t n, uint32_t tid
     }
 }
 
-// The most points a cell may hold for their ranks to be counted one against the others, which takes
-// the square of them: 8192 points in one cell 430 to 1200 us, in 64 cells 93. Past it the block sorts all of them
-// by cell and index: 63 and 69 us.
-constexpr uint32_t SG_RANK_MOST = 64;
+// Points are put in order within their cells by counting, for each, those of smaller index in its
+// cell, which takes the sum of the cells' squares; past SG_RANK_WORK times the sort's size the block sorts
+// all of them by cell and index. 8192 points in one cell: ranks 430 to 1200 us, sorted 63; in 64
+// cells 93 / 69; 5000 in 64 cells 30 / 48; 1000 in one 28 / 20.
+constexpr uint32_t SG_RANK_WORK = 72;
 static_assert(SMALL_N <= 1u << 13 && SMALL_CELLS <= 1u << 15, "a word holds cell and index");
 
 __global__ void __launch_bounds__(SG_T)
@@ -62,6 +66,7 @@ __global__ void __launch_bounds__(SG_T)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t s_warp[32];
     __shared__ uint32_t s_items;
+    __shared__ uint32_t s_work; // sum of the squares of the cells' points
     const uint32_t ncell = a.F.ncell, n = a.n;
     uint32_t* const start = reinterpret_cast<uint32_t*>(smem_raw); // [ncell + 1] counts, then offsets
     uint32_t* const where = start + ncell + 1;                     // [n] cell | rank << 16, then slot
@@ -71,7 +76,7 @@ __global__ void __launch_bounds__(SG_T)
     for (uint32_t c = tid; c <= ncell; c += SG_T)
         start[c] = 0;
     if (tid == 0)
-        s_items = 0;
+        s_items = s_work = 0;
     __syncthreads();
     const int dim[3] = {a.F.dim[0], a.F.dim[1], a.F.dim[2]};
     int off = 0;
@@ -104,17 +109,21 @@ __global__ void __launch_bounds__(SG_T)
         s_warp[lane] = warp_inclusive(w, lane) - w;
     }
     __syncthreads();
-    uint32_t at = incl - sum + s_warp[tid >> 5], most = 0;
+    uint32_t at = incl - sum + s_warp[tid >> 5], squares = 0;
     for (uint32_t c = c0; c < c1; ++c)
     {
         const uint32_t k = start[c];
         start[c] = at;
         at += k;
-        most = max(most, k);
+        squares += k * k;
     }
     if (tid == 0)
         start[ncell] = n;
-    const bool full = __syncthreads_or(a.sorted && most > SG_RANK_MOST);
+    squares = __reduce_add_sync(GR_FULL, squares);
+    if (lane == 0 && squares > 0)
+        atomicAdd(&s_work, squares);
+    __syncthreads();
+    const bool full = a.sorted && s_work > SG_RANK_WORK * sort_size(n);
     for (uint32_t c = tid; c <= ncell; c += SG_T)
         a.start[c] = start[c];
     for (uint32_t i = tid; i < n; i += SG_T)

@@ -1,4 +1,4 @@
-"""The one-block grid with cells of many points, past 64 of which the block sorts all points: lists
+"""The one-block grid with cells of many points, where the block sorts all points: lists
 against the oracle (a cell's points in index order are merged as sorted runs), sums that repeat to
 the bit, and the time of the grid, which grew with the square of a cell's points."""
 
@@ -17,9 +17,10 @@ def clusters(freud, n, cells):
     return box, (where + 0.4 * (rs.random_sample((n, 3)) - 0.5)).astype(np.float32)
 
 
-# about 64 points a cell is the limit; the sort has 64 words at least and any number of them
+# the sort has 64 words at least and any number of them; it is taken past 96 or 135 points in one cell, and of
+# 8192 points in some 114 cells and fewer
 @pytest.mark.parametrize("n, cells", [(1, 1), (63, 1), (64, 1), (65, 1), (66, 1), (127, 1), (129, 2), (450, 7), (640, 10),
-                                      (1000, 1), (1024, 9), (1025, 13), (4097, 40), (8191, 90), (8192, 500), (3000, 3)])
+                                      (1000, 1), (1024, 9), (1025, 13), (4097, 40), (8191, 90), (8192, 110), (8192, 120), (8192, 500), (96, 1), (97, 1), (135, 1), (136, 1), (3000, 3)])
 @pytest.mark.parametrize("by_distance", [False, True])
 def test_lists(freud, n, cells, by_distance):
     box, pts = clusters(freud, n, cells)
