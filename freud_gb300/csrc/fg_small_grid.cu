@@ -7,6 +7,7 @@
 #include "fg_prof.cuh"
 
 #include <algorithm>
+#include <atomic>
 
 namespace fg {
 
@@ -199,11 +200,17 @@ size_t small_grid_smem(uint32_t n, uint32_t ncell, bool sorted)
 void launch_small_grid(const SmallGrid& a, cudaStream_t s)
 {
     const size_t smem = small_grid_smem(a.n, a.F.ncell, a.sorted != 0);
-    // more than 48 KB, static arrays included, has to be allowed; always the same limit, so that
-    // threads do not lower each other's
-    if (smem > 47 * 1024)
+    // more than 48 KB, static arrays included, has to be allowed: once a device, for the largest grid
+    static std::atomic<uint64_t> allowed {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = uint64_t(1) << (dev & 63);
+    if (smem > 47 * 1024 && (allowed.load(std::memory_order_acquire) & bit) == 0)
+    {
         cudaFuncSetAttribute(k_small_grid, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(small_grid_smem(SMALL_N, SMALL_CELLS, true)));
+        allowed.fetch_or(bit, std::memory_order_release);
+    }
     ProfScope prof_("k_small_grid", s);
     k_small_grid<<<1, SG_T, smem, s>>>(a);
 }
