@@ -86,40 +86,31 @@ static cudaStream_t stream();
 class BlockCache
 {
 public:
-    // Size classes: powers of two up to 1 MB, then eighths of a power of two (an eighth
-    // at most is unused).
+    // Size classes: powers of two from 512 bytes to 1 MB, then eighths of a power of two (an
+    // eighth at most is unused).
     static size_t size_class(size_t n)
     {
-        size_t c = 512;
-        while (c < n && c < (size_t(1) << 20))
-            c <<= 1;
-        if (n <= c)
-            return c;
-        while (2 * c < n)
-            c <<= 1;
-        const size_t step = c / 8;
-        return (n + step - 1) / step * step;
+        return class_bytes(class_index(n));
     }
 
     void* take(size_t bytes, int dev, cudaStream_t s)
     {
         {
             std::lock_guard<std::mutex> lock(mu_);
-            for (const Key& key : {Key {dev, false, s, bytes}, Key {dev, true, nullptr, bytes}})
+            Device& d = device(dev);
+            for (Shelf* shelf : {find(dev, false, s), find(dev, true, nullptr)})
             {
-                auto it = free_.find(key);
-                if (it != free_.end() && !it->second.empty())
+                if (shelf == nullptr)
+                    continue;
+                std::vector<Block>& list = shelf->lists[class_index(bytes)];
+                if (!list.empty())
                 {
-                    void* p = it->second.back().p;
-                    it->second.pop_back();
-                    kept_[dev] -= bytes;
+                    void* p = list.back().p;
+                    list.pop_back();
+                    d.kept -= bytes;
                     return p;
                 }
             }
-        }
-        {
-            std::lock_guard<std::mutex> lock(mu_);
-            limit(dev);
         }
         void* p = nullptr;
         cudaError_t e = cudaMallocAsync(&p, bytes, s);
@@ -139,33 +130,20 @@ public:
         std::vector<void*> old;
         {
             std::lock_guard<std::mutex> lock(mu_);
-            const size_t most = limit(dev);
+            Device& d = device(dev);
+            Shelf& own = shelf(dev, false, s);
             // room by this stream's blocks and those of no stream; work of other streams may
             // still use theirs
-            while (kept_[dev] + bytes > most)
-            {
-                auto at = free_.end();
-                for (auto it = free_.begin(); it != free_.end(); ++it)
-                {
-                    const Key& k = it->first;
-                    if (!it->second.empty() && std::get<0>(k) == dev && (std::get<1>(k) || std::get<2>(k) == s) &&
-                        (at == free_.end() || it->second.front().released < at->second.front().released))
-                        at = it;
-                }
-                if (at == free_.end())
-                    break;
-                old.push_back(at->second.front().p);
-                at->second.erase(at->second.begin());
-                kept_[dev] -= std::get<3>(at->first);
-            }
-            if (kept_[dev] + bytes > most)
+            while (d.kept + bytes > d.limit && drop_oldest(own, find(dev, true, nullptr), d, old))
+                ;
+            if (d.kept + bytes > d.limit)
             {
                 old.push_back(p);
             }
             else
             {
-                free_[Key {dev, false, s, bytes}].push_back({p, ++clock_});
-                kept_[dev] += bytes;
+                own.lists[class_index(bytes)].push_back({p, ++clock_});
+                d.kept += bytes;
             }
         }
         for (void* q : old)
@@ -176,20 +154,23 @@ public:
     void leave(cudaStream_t s)
     {
         std::lock_guard<std::mutex> lock(mu_);
-        for (auto it = free_.begin(); it != free_.end();)
+        for (size_t k = 0; k < shelves_.size();)
         {
-            const Key k = it->first;
-            if (std::get<1>(k) || std::get<2>(k) != s)
+            if (shelves_[k]->idle || shelves_[k]->s != s)
             {
-                ++it;
+                ++k;
                 continue;
             }
-            auto& to = free_[Key {std::get<0>(k), true, nullptr, std::get<3>(k)}];
-            std::vector<Block> both(to.size() + it->second.size());
-            std::merge(to.begin(), to.end(), it->second.begin(), it->second.end(), both.begin(),
-                       [](const Block& x, const Block& y) { return x.released < y.released; });
-            to = std::move(both);
-            it = free_.erase(it);
+            Shelf& to = shelf(shelves_[k]->dev, true, nullptr); // (appended if new)
+            for (int c = 0; c < CLASSES; ++c)
+            {
+                std::vector<Block>&x = to.lists[c], &y = shelves_[k]->lists[c];
+                const size_t had = x.size();
+                x.insert(x.end(), y.begin(), y.end());
+                std::inplace_merge(x.begin(), x.begin() + had, x.end(),
+                                   [](const Block& l, const Block& r) { return l.released < r.released; });
+            }
+            shelves_.erase(shelves_.begin() + k);
         }
     }
 
@@ -199,18 +180,18 @@ public:
         std::vector<void*> blocks;
         {
             std::lock_guard<std::mutex> lock(mu_);
-            for (auto it = free_.begin(); it != free_.end();)
+            for (auto& shelf : shelves_)
             {
-                if (std::get<0>(it->first) != dev)
-                {
-                    ++it;
+                if (shelf->dev != dev)
                     continue;
+                for (auto& list : shelf->lists)
+                {
+                    for (const Block& b : list)
+                        blocks.push_back(b.p);
+                    list.clear();
                 }
-                for (const Block& b : it->second)
-                    blocks.push_back(b.p);
-                it = free_.erase(it);
             }
-            kept_[dev] = 0;
+            device(dev).kept = 0;
         }
         cudaDeviceSynchronize();
         for (void* p : blocks)
@@ -221,35 +202,118 @@ public:
     }
 
 private:
-    // device, of no stream, stream, bytes
-    using Key = std::tuple<int, bool, cudaStream_t, size_t>;
+    static constexpr int TOP = 11;                   // class of 1 MB
+    static constexpr int CLASSES = TOP + 1 + 8 * 44; // up to 2^64 bytes
     struct Block
     {
         void* p;
         uint64_t released;
     };
-
-    // Bytes kept of a device; its pool is told what to hold on to the first time (mu_ held).
-    size_t limit(int dev)
+    // The free lists of a stream (idle: of none); the front of a list was released longest ago.
+    struct Shelf
     {
-        auto it = limit_.find(dev);
-        if (it != limit_.end())
-            return it->second;
-        size_t left = 0, total = 0;
-        if (cudaMemGetInfo(&left, &total) != cudaSuccess)
-            total = 0;
-        cudaMemPool_t pool;
-        if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+        int dev;
+        bool idle;
+        cudaStream_t s;
+        std::array<std::vector<Block>, CLASSES> lists;
+    };
+    struct Device
+    {
+        bool known = false;
+        size_t kept = 0, limit = 0;
+    };
+
+    static int class_index(size_t n)
+    {
+        if (n <= (size_t(1) << 20))
         {
-            uint64_t hold = total / 2;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &hold);
+            int k = 0;
+            while ((size_t(512) << k) < n)
+                ++k;
+            return k;
         }
-        return limit_.emplace(dev, total / 4).first->second;
+        const int top = 63 - __builtin_clzll(n - 1); // 2^top < n <= 2^(top + 1)
+        return TOP + 1 + 8 * (top - 20) + static_cast<int>((n - 1 - (size_t(1) << top)) >> (top - 3));
+    }
+
+    static size_t class_bytes(int k)
+    {
+        return k <= TOP ? size_t(512) << k : size_t(9 + (k - TOP - 1) % 8) << (17 + (k - TOP - 1) / 8);
+    }
+
+    Shelf* find(int dev, bool idle, cudaStream_t s)
+    {
+        for (auto& shelf : shelves_)
+        {
+            if (shelf->dev == dev && shelf->idle == idle && shelf->s == s)
+                return shelf.get();
+        }
+        return nullptr;
+    }
+    Shelf& shelf(int dev, bool idle, cudaStream_t s)
+    {
+        Shelf* found = find(dev, idle, s);
+        if (found == nullptr)
+        {
+            shelves_.push_back(std::make_unique<Shelf>());
+            found = shelves_.back().get();
+            found->dev = dev;
+            found->idle = idle;
+            found->s = s;
+        }
+        return *found;
+    }
+
+    static bool drop_oldest(Shelf& own, Shelf* idle, Device& d, std::vector<void*>& old)
+    {
+        std::vector<Block>* at = nullptr;
+        size_t bytes = 0;
+        for (Shelf* shelf : {&own, idle})
+        {
+            for (int c = 0; shelf != nullptr && c < CLASSES; ++c)
+            {
+                std::vector<Block>& list = shelf->lists[c];
+                if (!list.empty() && (at == nullptr || list.front().released < at->front().released))
+                {
+                    at = &list;
+                    bytes = class_bytes(c);
+                }
+            }
+        }
+        if (at == nullptr)
+            return false;
+        old.push_back(at->front().p);
+        at->erase(at->begin());
+        d.kept -= bytes;
+        return true;
+    }
+
+    // What is kept of a device; its pool is told what to hold on to the first time.
+    Device& device(int dev)
+    {
+        if (devices_.size() <= static_cast<size_t>(dev))
+            devices_.resize(dev + 1);
+        Device& d = devices_[dev];
+        if (!d.known)
+        {
+            size_t left = 0, total = 0;
+            if (cudaMemGetInfo(&left, &total) != cudaSuccess)
+                total = 0;
+            d.limit = total / 4;
+            cudaMemPool_t pool;
+            if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess)
+            {
+                uint64_t hold = total / 2;
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &hold);
+            }
+            d.known = true;
+        }
+        return d;
     }
 
     std::mutex mu_;
-    std::map<Key, std::vector<Block>> free_; // the front was released longest ago
-    std::map<int, size_t> kept_, limit_;
+    std::vector<std::unique_ptr<Shelf>> shelves_; // one a thread or caller's stream in use
+    std::vector<Device> devices_;
     uint64_t clock_ = 0;
 };
 
