@@ -535,8 +535,9 @@ void hist_launch(const BatchGrid& g, const BallParams& p, const HistParams& h, c
 // can be counted (2 r_max below every box length, with room for the rounding), and along
 // each axis it is the smallest of |p - q|, |p - (q + L)| and |p - (q - L)|, each rounded as the
 // AABB arithmetic rounds it. About 35 warp instructions for 32 pairs, which costs less than
-// the latency of the grid, its groups and their tables up to SMALL_RDF_N points: whole calls
-// of 1000 points 78 us against 100, 3000 85 / 104, 5000 102 / 111.
+// the latency of the grid, its groups and their tables up to SMALL_RDF_N points at every r_max: whole
+// calls at density 1, r_max 0.4 to 6: 1000 points 81 to 84 us against 104 to 118, 3000 89 to 96 / 111
+// to 143, 5000 106 to 121 / 118 to 147.
 constexpr int SM_WARPS = 8;
 constexpr int SM_CHUNK = 64; // at most
 

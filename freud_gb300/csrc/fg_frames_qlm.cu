@@ -799,9 +799,9 @@ __global__ void __launch_bounds__(256)
 // A warp per particle: 32 points at a time are tested (the nearest image as in the small
 // histogram), the bonds listed, and then taken two a lane; the lanes' sums meet by shuffles.
 // Less than the latency of a grid and of groups whose lanes walk their bonds one after the
-// other: whole calls of l = 6, r_max 1.5, 1000 points at density 1 91 us against 144, 3000 132 /
-// 146, 4000 145 / 150, 5000 196 / 152; averaged 108 / 159, 147 / 194, 160 / 200, 212 / 201; l = 4, 6
-// 122 / 162, 190 / 196, 212 / 200 (2000 points: 148 / 170).
+// other: whole calls of l = 6 at density 1, r_max 1.2 to 3, 1000 points 98 to 101 us against 128 to
+// 326 by groups, 3000 137 to 141 / 141 to 320, 5000 206 to 217 / 160 to 323; averaged, r_max 1.2 to 2, 116
+// to 121 / 162 to 234, 153 to 156 / 171 to 281, 222 to 231 / 199 to 293. (fg_capi.cu has the rule.)
 constexpr int SQ_WARPS = 4;
 constexpr int SQ_LIST = 128; // listed bonds a warp
 
