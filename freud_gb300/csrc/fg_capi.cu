@@ -4329,6 +4329,7 @@ static SteinhardtTimes steinhardt_times(const StLs& ls, bool average, double n, 
         t.by_l += 7.1 * nl + bonds * orders * (0.27 + 2.2e-6 * n);
         t.arrays += 12.0 + 1.2e-6 * n * bonds * orders;
     }
+    t.arrays *= 1.12; // the others are kept to within the fits' spread
     return t;
 }
 
@@ -4548,9 +4549,9 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
         if (st->average)
         {
             // (in clusters, too, the averaging over bond arrays is the faster one)
-            precise = 1.12 * t.arrays < t.by_l;
+            precise = t.arrays < t.by_l;
         }
-        else if (1.12 * t.arrays + (F > 1 ? 80.0 : 20.0) < t.by_l)
+        else if (t.arrays + (F > 1 ? 80.0 : 20.0) < t.by_l)
         {
             // The fullest cell, read back, decides (12 to 20 us; with a batch, whose grid leaves the graph, 40): in a cluster the chain of its queries
             // is as long as the groups' or longer (1000 points in one cell, l = 4, 6, 8: by pairs 0.2 ms,
