@@ -177,6 +177,12 @@ struct StencilRows
     int segs; // runs a row: 1 when no x-cell of it lies across the boundary, else 3
 };
 
+// Cell of a bound, far from the integers' ends: bounds are infinite where a coordinate is.
+__device__ __forceinline__ int bound_cell(float v)
+{
+    return static_cast<int>(floorf(fminf(fmaxf(v, -1e6f), 1e6f)));
+}
+
 // (wide: half-width in place of the frame's shell.)
 __device__ __forceinline__ StencilRows stencil_rows(const FrameDesc& F, const GroupBox& gb, const GroupBounds& gd,
                                                     int wide = 0)
@@ -190,19 +196,19 @@ __device__ __forceinline__ StencilRows stencil_rows(const FrameDesc& F, const Gr
         // cell edges carry the rounding of the fractional coordinates (1e-3 of a cell is
         // far above it)
         const float r = gd.cull;
-        ya = max(ya, static_cast<int>(floorf((gd.lo[1] - r - F.b.lo[1]) * F.cells_per[1] - 1e-3f)));
-        yb = min(yb, static_cast<int>(floorf((gd.hi[1] + r - F.b.lo[1]) * F.cells_per[1] + 1e-3f)) + 1);
+        ya = max(ya, bound_cell((gd.lo[1] - r - F.b.lo[1]) * F.cells_per[1] - 1e-3f));
+        yb = min(yb, bound_cell((gd.hi[1] + r - F.b.lo[1]) * F.cells_per[1] + 1e-3f) + 1);
         if (!flat)
         {
-            za = max(za, static_cast<int>(floorf((gd.lo[2] - r - F.b.lo[2]) * F.cells_per[2] - 1e-3f)));
-            zb = min(zb, static_cast<int>(floorf((gd.hi[2] + r - F.b.lo[2]) * F.cells_per[2] + 1e-3f)) + 1);
+            za = max(za, bound_cell((gd.lo[2] - r - F.b.lo[2]) * F.cells_per[2] - 1e-3f));
+            zb = min(zb, bound_cell((gd.hi[2] + r - F.b.lo[2]) * F.cells_per[2] + 1e-3f) + 1);
         }
     }
     StencilRows R;
     R.y0 = ya;
-    R.ny = yb - ya;
+    R.ny = max(yb - ya, 0); // (none around an infinite coordinate)
     R.z0 = za;
-    R.n = R.ny * (zb - za);
+    R.n = R.ny * max(zb - za, 0);
     R.segs = gb.lo[0] >= s && gb.hi[0] + s <= F.dim[0] ? 1 : 3;
     return R;
 }
@@ -271,8 +277,8 @@ __device__ __forceinline__ StencilRuns stencil_runs(const FrameDesc& F, const Gr
             else
             {
                 const float r = sqrtf(gd.cull2 - g2);
-                xa = max(xa, static_cast<int>(floorf((gd.lo[0] - r - F.b.lo[0]) * F.cells_per[0] - 1e-3f)));
-                xb = min(xb, static_cast<int>(floorf((gd.hi[0] + r - F.b.lo[0]) * F.cells_per[0] + 1e-3f)));
+                xa = max(xa, bound_cell((gd.lo[0] - r - F.b.lo[0]) * F.cells_per[0] - 1e-3f));
+                xb = min(xb, bound_cell((gd.hi[0] + r - F.b.lo[0]) * F.cells_per[0] + 1e-3f));
             }
         }
         bool mine = true, own_row = false;
