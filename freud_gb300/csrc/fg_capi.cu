@@ -1172,6 +1172,14 @@ struct NlPlan
 // lanes over candidates only.
 static int g_count_kernel = 0;
 
+// Candidates that fit a group of met expected ones.
+int nl_room(double met)
+{
+    const double most = met + 5.0 * std::sqrt(met);
+    return most <= 256.0 ? 256 : (most <= 512.0 ? 512 : (most <= 768.0 ? 768 : 1024));
+}
+constexpr uint32_t NL_WIDE = 1u << 22; // points from which on the sort keys have 64 bits
+
 // The grid of a ball query over query groups: cells of half r_max, at least two an axis, and
 // boxes whose groups have at most 900 candidates (of uniform points). False where there is
 // none or the block-per-cell kernels are the faster ones: a group is one warp's chain of
@@ -1179,7 +1187,9 @@ static int g_count_kernel = 0;
 // query, groups against blocks: 1600 cells (25k points, r_max 2.5) 264 against 250 us, 3200:
 // 284 / 306, 6400: 357 / 420; r_max 1.5 and 4200 cells 226 / 242, 35000 cells 270 / 580. The
 // dense cells of the 4096-candidate kernels (one block an SM) ten times earlier: 125 cells
-// 263 / 234, 216: 272 / 272, 343: 272 / 301, 1331: 315 / 488.
+// 263 / 234, 216: 272 / 272, 343: 272 / 301, 1331: 315 / 488. From 2^22 points on the sort keys are of 64
+// bits, and groups of more than 512 candidates lose to blocks where those are not of the dense kind (4.3M
+// points, wrap, r_max 2.8 12.0 / 9.6 ms, 3.0 12.5 / 10.0, 3.3 (dense) 15.4 / 25.3, 2.6 (512) 7.9 / 9.6).
 bool nl_group_grid(const fg_nq* nq, const fg_query_args& a, uint32_t nqp, FrameDesc& F, double& groups, double& met)
 {
     const HostBox& hb = nq->box;
@@ -1190,7 +1200,8 @@ bool nl_group_grid(const fg_nq* nq, const fg_query_args& a, uint32_t nqp, FrameD
     grid_dims(hb, a.r_max * (1.0f + 1e-5f), nq->n, dim);
     DevGrid coarse {};
     coarse.ncell = dim[0] * dim[1] * dim[2];
-    if (coarse.ncell * (cell_cap_for(coarse, nq->n, flat) > CELL_CAP ? 10 : 1) < 2500)
+    const bool dense = cell_cap_for(coarse, nq->n, flat) > CELL_CAP;
+    if (coarse.ncell * (dense ? 10 : 1) < 2500)
         return false;
     grid_dims(hb, a.r_max * 0.5f * (1.0f + 1e-5f), nq->n, dim);
     if (dim[0] < 2 || dim[1] < 2 || (!flat && dim[2] < 2))
@@ -1198,6 +1209,8 @@ bool nl_group_grid(const fg_nq* nq, const fg_query_args& a, uint32_t nqp, FrameD
     const double cell = box_volume(hb) / (static_cast<double>(dim[0]) * dim[1] * dim[2]);
     F = frame_desc(hb, dim, 2);
     groups = nl_boxes(dim, nqp, nq->n, a.r_max / (flat ? std::sqrt(cell) : std::cbrt(cell)), F.nb, &met);
+    if (nq->n >= NL_WIDE && nl_room(met) > 512 && !dense)
+        return false;
     return met > 0.0;
 }
 
@@ -1214,10 +1227,9 @@ bool plan_nl_groups(fg_nq* nq, const float* dq, uint32_t nqp, const fg_query_arg
     double met = 0.0, groups = 0.0;
     if (!nl_group_grid(nq, a, nqp, P.F, groups, met))
         return false;
-    const double most = met + 5.0 * std::sqrt(met);
-    P.room = most <= 256.0 ? 256 : (most <= 512.0 ? 512 : (most <= 768.0 ? 768 : 1024));
+    P.room = nl_room(met);
     P.wrap = wrap;
-    P.wide = nq->n >= (1u << 22);
+    P.wide = nq->n >= NL_WIDE;
     P.expected = static_cast<uint32_t>(groups) + 1;
     P.F.n = nqp;
     float pd[3];
