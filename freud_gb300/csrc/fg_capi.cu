@@ -4341,7 +4341,7 @@ static SteinhardtTimes steinhardt_times(const StLs& ls, bool average, double n, 
         t.by_l += 7.1 * nl + bonds * orders * (0.27 + 2.2e-6 * n);
         t.arrays += 12.0 + 1.2e-6 * n * bonds * orders;
     }
-    t.arrays *= 1.12; // the others are kept to within the fits' spread
+    t.arrays *= 1.04; // (the others where the fits tell no difference)
     return t;
 }
 
@@ -4528,8 +4528,7 @@ static void steinhardt_frames(fg_steinhardt* st, fg_frames* fr, const fg_query_a
     }
     std::vector<double> sys(2 * static_cast<size_t>(F) * stride);
     // Up to six l of at most 12 without wl (its harmonics are float-float) go the way that comes out
-    // cheapest (steinhardt_times), bond arrays only where they do by an eighth: within 1 % of the
-    // best of the three on average. 2000 points,
+    // cheapest (steinhardt_times), within 1 % of the best of the three on average. 2000 points,
     // averaged, r_max 1.5: l = 6 by pairs 134 us, by l 169, arrays 199; l = 4, 6, 8, 10 287, 378, 227;
     // 200,000 points, l = 4, 6, 8: by l 740, arrays 899; 5000 points, r_max 2.5, l = 2, 4, .., 12:
     // by l 1490, arrays 730. Pairs are taken up to a fifth above the others where nothing is averaged: their time does
